@@ -32,7 +32,7 @@ LAWKW = {
 }
 LAWS = ("linear", "bilinear", "trilinear", "exponential")
 RATE = -1e-11       # metres per step at the loaded nodes: quasi-static, elastic over a run of these cases
-RATE32 = -5e-10     # the FP32 form's: its force rounding is absolute, it is used at larger displacements
+RATE32 = -5e-9      # the FP32 form's, at 2.5 mm spacing: its force rounding is absolute, it is used at larger displacements
 BREAK_RATE = -1e-7  # the rate that takes a beam of 20 nodes depth at 5 mm past its peak in about 1 200 steps
 
 
@@ -117,11 +117,15 @@ def draw(rng):
 
 # ---- what a program has in hand before the call ----
 
+def _rate(case):
+    return RATE32 * case["dx"] / 2.5e-3 if case.get("prec") == "fp32" else RATE
+
+
 def _beam(case, seed):
     """Host arrays of the case's beam for this seed, and the loading rate."""
     rng = np.random.default_rng(seed)
     E = 37e9 * (1 + 0.05 * rng.standard_normal())
-    rate = (RATE32 if case.get("prec") == "fp32" else RATE) * (1 + 0.05 * rng.standard_normal())
+    rate = _rate(case) * (1 + 0.05 * rng.standard_normal())
     nx, dx = case["nx"], case["dx"]
     kw = {}
     if case.get("notch"):   # between two node planes, right of midspan, 0.4 of the depth
@@ -158,7 +162,7 @@ def prepare(case, seed):
         return dict(case=case, s=s)
     if kind == "batch":
         rng = np.random.default_rng(seed)
-        rate = (RATE32 if case["prec"] == "fp32" else RATE) * (1 + 0.05 * rng.standard_normal())
+        rate = _rate(case) * (1 + 0.05 * rng.standard_normal())
         members = []
         for sp, law in bb.beam.size_effect_series(case["members"], depth_range=(0.05, case["depth"]), dx=case["dx"]):
             sp.seed = int(rng.integers(1 << 30))   # the depths stay, the material is drawn anew
