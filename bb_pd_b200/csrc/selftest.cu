@@ -4,7 +4,9 @@
 #include "divide.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <vector>
 
 using namespace bbpd;
 
@@ -72,6 +74,53 @@ __global__ void division_selftest_kernel(int64_t n, uint64_t seed, Counts *c)
     atomicAdd(&c->skipped, sk);
     atomicAdd(&c->samples, cnt);
     atomicMax(&c->rcp_err_bits, (unsigned long long)__double_as_longlong(maxerr));
+}
+
+struct SqrtCounts {
+    unsigned long long sqrt_bad, recip_bad, samples, seed_err_bits;
+};
+
+__device__ __forceinline__ void sqrt_check(double x, unsigned long long &sb, unsigned long long &rb,
+                                           unsigned long long &cnt, double &seed_err)
+{
+    double L, rL;
+    bool ok;
+    sqrt_recip_rn(x, L, rL, ok);
+    if (!ok) return;
+    cnt++;
+    const double ref = sqrt(x);
+    seed_err = fmax(seed_err, fabs(rsqrt_approx(x) * ref - 1.0));
+    if (__double_as_longlong(L) != __double_as_longlong(ref)) sb++;
+    if (__double_as_longlong(rL) != __double_as_longlong(1.0 / ref)) rb++;
+}
+
+// sqrt_recip_rn against IEEE sqrt and division: the hard significands, every
+// high word of [1, 4) with three low words, and n seeded samples (any
+// significand, exponents -300 .. 300 and often near squared bond lengths).
+__global__ void sqrt_selftest_kernel(const double *hard, int64_t nhard, int64_t n, uint64_t seed, SqrtCounts *c)
+{
+    unsigned long long sb = 0, rb = 0, cnt = 0;
+    double err = 0;
+    const int64_t nhigh = (int64_t)1 << 21, all = nhard + 3 * nhigh + n;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < all; t += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t h1 = mix64(seed ^ (uint64_t)t * 0xD1B54A32D192ED03ull), h2 = mix64(h1);
+        double x;
+        if (t < nhard) {
+            x = hard[t];
+        } else if (t < nhard + 3 * nhigh) {
+            const int64_t q = t - nhard, w = q % nhigh;
+            const uint64_t low = q < nhigh ? 0 : q < 2 * nhigh ? 0xFFFFFFFFull : (h1 & 0xFFFFFFFFull);
+            x = __longlong_as_double((long long)((((uint64_t)1023 << 20) + (uint64_t)w) << 32 | low));
+        } else {
+            const int e = (h2 >> 63) ? (int)((h2 >> 40) % 40) - 30 : (int)((h2 >> 40) % 601) - 300;
+            x = make_double(h1, e);
+        }
+        sqrt_check(x, sb, rb, cnt, err);
+    }
+    atomicAdd(&c->sqrt_bad, sb);
+    atomicAdd(&c->recip_bad, rb);
+    atomicAdd(&c->samples, cnt);
+    atomicMax(&c->seed_err_bits, (unsigned long long)__double_as_longlong(err));
 }
 
 // Uniform doubles in [lo, hi) from a counter (splitmix64), the sampler of the
@@ -176,6 +225,63 @@ extern "C" int bbpd_selftest_exp(double lo, double hi, int64_t n, uint64_t seed,
     if (e != cudaSuccess) return fail(BBPD_ERR_CUDA, "exp selftest: %s", cudaGetErrorString(e));
     *fast_vs_accurate = (int64_t)h[0];
     *bits_sum = (uint64_t)h[1];
+    return BBPD_OK;
+}
+
+// Every double in [1, 4) whose square root lies next to a rounding midpoint
+// M 2^-53 (M odd, 54 bits) with |M^2 - x scaled| < 2^13: the roots M of
+// M^2 = c mod 2^54 (x in [1, 2)) or 2^55 (x in [2, 4)), lifted bit by bit.
+static std::vector<double> hard_sqrt_arguments()
+{
+    std::vector<double> out;
+    for (int64_t c = -(1 << 13) + 1; c < (1 << 13); c += 8) {   // c = 1 mod 8
+        for (int k = 54; k <= 55; k++) {
+            const uint64_t mask = ((uint64_t)1 << k) - 1;
+            uint64_t r = 1;
+            for (int j = 3; j < k; j++)
+                if (((r * r - (uint64_t)c) >> j) & 1) r += (uint64_t)1 << (j - 1);
+            const uint64_t half = (uint64_t)1 << (k - 1);
+            for (uint64_t M : {r & mask, (0 - r) & mask, (r + half) & mask, (half - r) & mask}) {
+                if (M < ((uint64_t)1 << 53) || M >= ((uint64_t)1 << 54)) continue;
+                const __int128 sq = (__int128)M * M - c;
+                if (sq & (((__int128)1 << k) - 1)) continue;
+                const __int128 X = sq >> k;
+                if (X < ((__int128)1 << 52) || X >= ((__int128)1 << 53)) continue;
+                out.push_back(std::ldexp((double)(int64_t)X, k == 54 ? -52 : -51));
+            }
+        }
+    }
+    return out;
+}
+
+extern "C" int bbpd_selftest_sqrt(int64_t n, uint64_t seed, int64_t *sqrt_mismatches, int64_t *recip_mismatches,
+                                  int64_t *hard_cases, int64_t *samples, double *rsqrt_approx_max_relerr)
+{
+    int rc = require_device();
+    if (rc) return rc;
+    if (n < 0 || !sqrt_mismatches || !recip_mismatches || !hard_cases || !samples || !rsqrt_approx_max_relerr)
+        return fail(BBPD_ERR_ARG, "bad argument");
+    const std::vector<double> hard = hard_sqrt_arguments();
+    double *dh = nullptr;
+    SqrtCounts *dc = nullptr;
+    BBPD_CUDA_TRY(cudaMalloc(&dh, sizeof(double) * hard.size()));
+    cudaError_t e = cudaMalloc(&dc, sizeof(SqrtCounts));
+    SqrtCounts h{};
+    if (e == cudaSuccess) e = cudaMemset(dc, 0, sizeof(SqrtCounts));
+    if (e == cudaSuccess) e = cudaMemcpy(dh, hard.data(), sizeof(double) * hard.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        sqrt_selftest_kernel<<<148 * 8, 256>>>(dh, (int64_t)hard.size(), n, seed, dc);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&h, dc, sizeof(SqrtCounts), cudaMemcpyDeviceToHost);
+    cudaFree(dh);
+    cudaFree(dc);
+    if (e != cudaSuccess) return fail(BBPD_ERR_CUDA, "sqrt selftest: %s", cudaGetErrorString(e));
+    *sqrt_mismatches = (int64_t)h.sqrt_bad;
+    *recip_mismatches = (int64_t)h.recip_bad;
+    *hard_cases = (int64_t)hard.size();
+    *samples = (int64_t)h.samples;
+    std::memcpy(rsqrt_approx_max_relerr, &h.seed_err_bits, 8);
     return BBPD_OK;
 }
 

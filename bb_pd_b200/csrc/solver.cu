@@ -570,16 +570,16 @@ __device__ __forceinline__ double3 entry_force(const Dev &d, int64_t e, const Fe
     const double s0b = d.s0e ? __ldg(d.s0e + e) : d.P.s0;
     double3 r;
     {
-        // calculatedeformedlengthMex.c:37-43 with its division by L0 and the
+        // calculatedeformedlengthMex.c:37-43 with its square root, division by L0 and the
         // three of calculatebondforcesMex.c:34-36 by L done as correctly
         // rounded quotients with shared reciprocals (divide.cuh): bit-identical
         // to IEEE division whenever `safe` holds.
         const double dX = f.xj - xi, dY = f.yj - yi, dZ = f.zj - zi;
-        const double L = sqrt(dX * dX + dY * dY + dZ * dZ);
-        const double s = quot_rn(L - f.g.l0, f.g.l0, f.g.rl0);
+        double L, rL;
         bool okr;
-        const double rL = recip_rn(L, okr);
-        if (safe && okr && f.sv == 0 && f.g.rl0 > 0 && L > 0 &&
+        sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
+        const double s = quot_rn(L - f.g.l0, f.g.l0, f.g.rl0);
+        if (safe && okr && f.sv == 0 && f.g.rl0 > 0 &&
             law_quiet<LAW>(d.P, bt, s, s0b, f.sc)) {
             const double t = ((f.g.bs * s) * d.V) * f.g.vcf;
             r.x = t * quot_rn(dX, L, rL);
@@ -650,11 +650,11 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
             const double s0b = d.s0e ? __ldg(d.s0e + e0 + q) : d.P.s0;
             const int bt = (w >> BT_SHIFT) & 3;
             const double dX = xj[q] - xi, dY = yj[q] - yi, dZ = zj[q] - zi;
-            const double L = sqrt(dX * dX + dY * dY + dZ * dZ);
-            const double s = quot_rn(L - g.l0, g.l0, g.rl0);
+            double L, rL;
             bool okr;
-            const double rL = recip_rn(L, okr);
-            const bool fast = safe && okr && sv == 0 && g.rl0 > 0 && L > 0 && law_quiet<LAW>(d.P, bt, s, s0b, scv);
+            sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
+            const double s = quot_rn(L - g.l0, g.l0, g.rl0);
+            const bool fast = safe && okr && sv == 0 && g.rl0 > 0 && law_quiet<LAW>(d.P, bt, s, s0b, scv);
             const double t = ((g.bs * s) * d.V) * g.vcf;
             fx[q] = t * quot_rn(dX, L, rL);
             fy[q] = t * quot_rn(dY, L, rL);
@@ -1504,11 +1504,11 @@ __device__ __forceinline__ void lattice_forces(const Dev &d, int n, bool valid, 
             else gd = ldg_dict(d.dict, c);
             const double scv = SCE ? __ldcs(d.sce + (t.y + n + t.z)) : d.P.sc;
             const int bt = (sv >> LST_BT_SHIFT) & 3;
-            const double L = sqrt(dX * dX + dY * dY + dZ * dZ);
-            const double s = quot_rn(L - gd.l0, gd.l0, gd.rl0);
+            double L, rL;
             bool okr;
-            const double rL = recip_rn(L, okr);
-            const bool fast = safe && okr && (sv & ST_MASK) == 0 && gd.rl0 > 0 && L > 0 &&
+            sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
+            const double s = quot_rn(L - gd.l0, gd.l0, gd.rl0);
+            const bool fast = safe && okr && (sv & ST_MASK) == 0 && gd.rl0 > 0 &&
                               law_quiet<LAW>(d.P, bt, s, d.P.s0, scv);
             const double tt = ((gd.bs * s) * d.V) * gd.vcf;
             fx[q] = tt * quot_rn(dX, L, rL);

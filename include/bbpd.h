@@ -599,6 +599,16 @@ int bbpd_selftest_division(int64_t n, uint64_t seed, int64_t *recip_mismatches,
                            int64_t *quot_mismatches, int64_t *samples,
                            double *rcp_approx_max_relerr);
 
+/* Diagnostic: compares the kernels' branch-free square root and its reciprocal
+ * (Goldschmidt's iteration, divide.cuh) with IEEE sqrt and division on the
+ * device, bit for bit: on the arguments whose square roots lie next to a
+ * rounding midpoint (hard_cases of them), on every high word of [1, 4) and on n
+ * seeded samples; also the largest relative error of the hardware
+ * reciprocal-square-root approximation. */
+int bbpd_selftest_sqrt(int64_t n, uint64_t seed, int64_t *sqrt_mismatches,
+                       int64_t *recip_mismatches, int64_t *hard_cases, int64_t *samples,
+                       double *rsqrt_approx_max_relerr);
+
 /* Diagnostic: the device's correctly rounded exp (the exponential law's exp,
  * in place of CUDA's, so that the law rounds like the reference's libm call,
  * calculatebsfexponentialMex.c:43) on n samples uniform in [lo, hi) drawn

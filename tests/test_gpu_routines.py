@@ -208,6 +208,21 @@ def test_division_selftest():
     assert rb.value == 0 and qb.value == 0, (rb.value, qb.value)
 
 
+def test_sqrt_selftest():
+    """The kernels' branch-free square root and reciprocal (Goldschmidt) equal
+    IEEE sqrt and division bit for bit: the arguments next to rounding
+    midpoints, every high word, and 2e8 seeded samples."""
+    import ctypes as C
+    sb, rb, hard, n = C.c_int64(), C.c_int64(), C.c_int64(), C.c_int64()
+    err = C.c_double()
+    bb._native.check(bb._native.lib().bbpd_selftest_sqrt(C.c_int64(200_000_000), C.c_uint64(20261205), C.byref(sb),
+                                                          C.byref(rb), C.byref(hard), C.byref(n), C.byref(err)))
+    print(f"samples {n.value}, hard {hard.value}, rsqrt.approx max rel err {err.value:.3e}")
+    assert hard.value > 2000 and n.value > 200_000_000
+    assert err.value < 2.0 ** -18   # two rounds of 1.5 err^2 stay below 2^-60
+    assert sb.value == 0 and rb.value == 0, (sb.value, rb.value)
+
+
 def test_damage_vs_oracle():
     inp = bb.beam.build(bb.beam.small(nx=20, ny=4, nz=6))
     bl, nfam = inp["BONDLIST"], inp["nFAMILYMEMBERS"]
