@@ -68,6 +68,7 @@ namespace {
 constexpr uint32_t COL_MASK = 0x00FFFFFFu;
 constexpr uint32_t F_CHUNK = 1u << 24;   // first entry of a new OpenMP chunk in this list
 constexpr int BT_SHIFT = 25;             // bits 25-26: BONDTYPE
+constexpr uint32_t BT_BITS = 3u << BT_SHIFT;
 constexpr uint8_t ST_BROKEN = 1;         // fail == 0
 constexpr uint8_t ST_SOFT = 2;           // flagBondSoftening == 1
 constexpr uint8_t ST_DAMAGED = 4;        // BSF != +0.0 (BSF stored in bsf[])
@@ -143,6 +144,8 @@ struct Dev {
     const double *s0e, *s1e, *sce;   // per-entry law stretches or null
     double s0q;                      // FP32 fast path's s0: the scalar s0, or the least per-entry s0
                                      // (entries above it take the general path, which reads their own)
+    int quiet_hi;                    // FP64 fast path: a stretch whose high word (as a signed number) is below this
+                                     // is below the law's stretch, whatever the bond (see quiet_high_word)
     double *smax;                    // damage-energy tracking: largest stretch of each concrete entry past s0, or null
     const double *X;
     double *xb0, *xb1;               // positions: step n reads xb[(n-1)&1], writes xb[n&1]
@@ -490,6 +493,20 @@ __device__ __forceinline__ bool law_quiet(const LawScalars &P, int bt, double s,
     return !(bt == 0 && s > s0);
 }
 
+// High word below which a stretch is certainly not above x: for x >= 0 the
+// high words of finite doubles s <= 0 or s < x compare like signed integers. A
+// stretch that shares x's high word counts as active and takes the general
+// path, which tests exactly, and so does every stretch when x is negative; a
+// NaN x keeps every entry quiet, as `s > NaN` does.
+inline int quiet_high_word(double x)
+{
+    if (std::isnan(x)) return INT32_MAX;
+    if (x < 0) return INT32_MIN;
+    uint64_t b;
+    std::memcpy(&b, &x, 8);
+    return (int)(b >> 32) & 0x7FFFFFFF;
+}
+
 // One entry in full generality: law, damage state written back when it
 // changes, bond force with the NaN guards of calculatebondforcesMex.c. Kept
 // out of line: intact bonds whose law is quiet never come here.
@@ -613,6 +630,62 @@ __device__ __forceinline__ void load_pos(const double4 *p, double &x, double &y,
     (void)w;
 }
 
+// FP64 form, the fast path of one group of 4 entries of a lane at (xi, yi, zi):
+// without branches, so that the four dependency chains interleave. Returns the
+// mask of the slots that need the general path. Slots past the lane's list are
+// layout padding (all streams zero): they name node 0 and dictionary entry 0,
+// so every slot gathers a valid record and needs no select.
+template <int LAW, class CID, int SCE>
+__device__ __forceinline__ unsigned group_fast(const Dev &d, const Group<CID> &G, int64_t e0, bool safe,
+                                               const double4 *xa, double xi, double yi, double zi,
+                                               double (&fx)[4], double (&fy)[4], double (&fz)[4])
+{
+    double xj[4], yj[4], zj[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t j = group_w(G, q) & COL_MASK;
+        load_pos(xa + j, xj[q], yj[q], zj[q]);
+    }
+    unsigned fast = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t w = group_w(G, q);
+        const DictEntry g = ldg_dict(d.dict, G.cid(q));
+        const double dX = xj[q] - xi, dY = yj[q] - yi, dZ = zj[q] - zi;
+        double L, rL;
+        bool okr;
+        sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
+        const double s = quot_rn(L - g.l0, g.l0, g.rl0);
+        const double t = ((g.bs * s) * d.V) * g.vcf;
+        fx[q] = t * quot_rn(dX, L, rL);
+        fy[q] = t * quot_rn(dY, L, rL);
+        fz[q] = t * quot_rn(dZ, L, rL);
+        // tests on high words and without short circuits: no branch, no FP64
+        const bool intact = (G.s & (0xFFu << (8 * q))) == 0, regular = __double2hiint(g.rl0) >= 0;
+        bool quiet;
+        if (LAW == BBPD_LAW_LINEAR && SCE != 0) {
+            const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
+            quiet = law_quiet<LAW>(d.P, (w >> BT_SHIFT) & 3, s, 0.0, scv);
+        } else {
+            quiet = (__double2hiint(s) < d.quiet_hi) | (LAW != BBPD_LAW_LINEAR && (w & BT_BITS) != 0);
+        }
+        fast |= (okr & intact & regular & quiet ? 1u : 0u) << q;
+    }
+    return safe ? ~fast : ~0u;
+}
+
+// The general path of slot q of a group.
+template <int LAW, int PREC, class CID, int SCE>
+__device__ __forceinline__ double3 group_slow(const Dev &d, const Group<CID> &G, int q, int64_t e0, const double *xs,
+                                              double xi, double yi, double zi)
+{
+    const int64_t nN = d.n_nodes;
+    const uint32_t w = group_w(G, q), j = w & COL_MASK;
+    const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
+    return entry_general<LAW, PREC>(d, e0 + q, w, (G.s >> (8 * q)) & 0xFFu, ldg_dict(d.dict, G.cid(q)), scv, xi, yi,
+                                    zi, xs[j], xs[j + nN], xs[j + 2 * nN]);
+}
+
 // Forces of the 32 nodes of one slice (FP64 form).
 // Lane `lane` owns node sl*32+lane and walks its entries in bond order, a group
 // of 4 at a time: the next group's streams load while the current group's 12
@@ -627,10 +700,9 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
     const int64_t i = sl * 32 + lane;
     const int dg = (i < nN) ? d.deg[i] : 0;
     const int64_t sb = d.slice_ptr[sl];
-    const double *x0 = xs, *x1 = xs + nN, *x2 = xs + 2 * nN;
 
     double xi = 0, yi = 0, zi = 0;
-    if (i < nN) { xi = x0[i]; yi = x1[i]; zi = x2[i]; }
+    if (i < nN) { xi = xs[i]; yi = xs[i + nN]; zi = xs[i + 2 * nN]; }
     tx = 0.0; ty = 0.0; tz = 0.0;
     double ax = 0.0, ay = 0.0, az = 0.0;
 
@@ -642,42 +714,11 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
         if (g + kPrefetch < ng) prefetch_group<CID, SCE>(d, e0 + 128 * kPrefetch);
         if (g + 1 < ng) load_group<CID>(d, e0 + 128, Gn);
         const int nq = min(4, dg - 4 * g);
-        // Slots past the lane's list are layout padding (all streams zero):
-        // they name node 0 and dictionary entry 0, so every slot gathers a
-        // valid record and the pass below needs no per-slot selects.
-        double xj[4], yj[4], zj[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t j = group_w(Gc, q) & COL_MASK;
-            load_pos(xa + j, xj[q], yj[q], zj[q]);
-        }
-        // pass 1: the fast path of all entries of the group, without
-        // branches, so that the four dependency chains interleave
         double fx[4], fy[4], fz[4];
-        unsigned slow = 0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const bool valid = q < nq;
-            const uint32_t w = group_w(Gc, q), c = Gc.cid(q), sv = (Gc.s >> (8 * q)) & 0xFFu;
-            const DictEntry g = ldg_dict(d.dict, c);
-            const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
-            const double s0b = d.s0e ? __ldg(d.s0e + e0 + q) : d.P.s0;
-            const int bt = (w >> BT_SHIFT) & 3;
-            const double dX = xj[q] - xi, dY = yj[q] - yi, dZ = zj[q] - zi;
-            double L, rL;
-            bool okr;
-            sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
-            const double s = quot_rn(L - g.l0, g.l0, g.rl0);
-            const bool fast = safe && okr && sv == 0 && g.rl0 > 0 && law_quiet<LAW>(d.P, bt, s, s0b, scv);
-            const double t = ((g.bs * s) * d.V) * g.vcf;
-            fx[q] = t * quot_rn(dX, L, rL);
-            fy[q] = t * quot_rn(dY, L, rL);
-            fz[q] = t * quot_rn(dZ, L, rL);
-            if (valid && !fast) slow |= 1u << q;
-        }
-        // pass 2: the sum in the reference's order. A full group with no
-        // general entry and no chunk start (nearly every group) adds its four
-        // forces straight; otherwise each entry is taken in turn.
+        const unsigned slow = group_fast<LAW, CID, SCE>(d, Gc, e0, safe, xa, xi, yi, zi, fx, fy, fz) & ((1u << nq) - 1);
+        // the sum in the reference's order: a full group with no general entry
+        // and no chunk start (nearly every group) adds its four forces
+        // straight; otherwise each entry is taken in turn
         const uint32_t chunk = (Gc.w.x | Gc.w.y | Gc.w.z | Gc.w.w) & F_CHUNK;
         if (nq == 4 && (slow | chunk) == 0) {
 #pragma unroll
@@ -688,15 +729,9 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (q < nq) {
-                const uint32_t w = group_w(Gc, q);
                 double3 r = make_double3(fx[q], fy[q], fz[q]);
-                if (slow & (1u << q)) {
-                    const uint32_t j = w & COL_MASK;
-                    const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
-                    r = entry_general<LAW, PREC>(d, e0 + q, w, (Gc.s >> (8 * q)) & 0xFFu,
-                                                 ldg_dict(d.dict, Gc.cid(q)), scv, xi, yi, zi, x0[j], x1[j], x2[j]);
-                }
-                if (w & F_CHUNK) {  // partial of the previous OpenMP thread is complete
+                if (slow & (1u << q)) r = group_slow<LAW, PREC, CID, SCE>(d, Gc, q, e0, xs, xi, yi, zi);
+                if (group_w(Gc, q) & F_CHUNK) {  // partial of the previous OpenMP thread is complete
                     tx = tx + ax; ty = ty + ay; tz = tz + az;
                     ax = 0.0; ay = 0.0; az = 0.0;
                 }
@@ -731,6 +766,71 @@ __device__ __forceinline__ double3 entry_general_x(const Dev &d, int64_t e, uint
 // FP64 in the reference's order. Bonds whose stretch lies within the guard band
 // of the critical stretch, damaged or broken bonds and bonds whose law is active
 // take the general path with FP64 positions.
+//
+// The fast path of one group, without branches; returns the mask of the slots
+// that need the general path. Padding slots name node 0 and dictionary entry 0
+// (see group_fast).
+template <int LAW, class CID, int SCE>
+__device__ __forceinline__ unsigned group_fast_x(const Dev &d, const Group<CID> &G, int64_t e0, const float4 *urh,
+                                                 const float2 *url, float4 ui, float2 li, float (&fx)[4],
+                                                 float (&fy)[4], float (&fz)[4])
+{
+    const float s0f = (float)d.s0q, guardf = (float)d.guard, scf0 = (float)d.P.sc;
+    const float steelf = (float)d.P.sc_steel;
+    float4 uj[4];
+    float2 lj[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t j = group_w(G, q) & COL_MASK;
+        uj[q] = urh[j];
+        lj[q] = url[j];
+    }
+    unsigned slow = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t w = group_w(G, q), c = G.cid(q), sv = (G.s >> (8 * q)) & 0xFFu;
+        const int bt = (w >> BT_SHIFT) & 3;
+        float4 A, Bv;
+        ldg_dictx(d.dictx, c, A, Bv);
+        const float etx = (uj[q].x - ui.x) + (uj[q].w - ui.w);
+        const float ety = (uj[q].y - ui.y) + (lj[q].x - li.x);
+        const float etz = (uj[q].z - ui.z) + (lj[q].y - li.y);
+        const float ex = A.x + etx, ey = A.y + ety, ez = A.z + etz;
+        const float L2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
+        const float rL = rsqrtf(L2);
+        const float L = L2 * rL;
+        const float num = __fmaf_rn(etz, A.z + ez, __fmaf_rn(ety, A.y + ey, __fmaf_rn(etx, A.x + ex, Bv.y)));
+        const float sf = __fdividef(num, A.w * (L + A.w));
+        // Fast iff the law is quiet and sf is outside the guard band round
+        // the critical stretch (band edges rounded outwards); a NaN
+        // stretch (zero, infinite or NaN length) fails every comparison.
+        const float scf = has_sce<SCE>(d) ? (float)__ldcs(d.sce + e0 + q) : scf0;
+        bool fast;
+        if (LAW == BBPD_LAW_LINEAR) {
+            const float critf = (bt == 0) ? scf : (bt == 1 ? 3.f * scf : steelf);
+            fast = sf <= __fsub_rd(critf, guardf);
+        } else {
+            const float top = (bt == 0) ? s0f : INFINITY;
+            fast = sf <= top && (sf <= __fsub_rd(scf, guardf) || sf >= __fadd_ru(scf, guardf));
+        }
+        fast = fast && sv == 0 && Bv.z != 0.f;
+        const float qf = Bv.x * sf * rL;
+        fx[q] = qf * ex;
+        fy[q] = qf * ey;
+        fz[q] = qf * ez;
+        if (!fast) slow |= 1u << q;
+    }
+    return slow;
+}
+
+template <int LAW, class CID, int SCE>
+__device__ __forceinline__ double3 group_slow_x(const Dev &d, const Group<CID> &G, int q, int64_t e0, int64_t i,
+                                                const double *xs)
+{
+    const double scd = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
+    return entry_general_x<LAW>(d, e0 + q, group_w(G, q), (G.s >> (8 * q)) & 0xFFu, G.cid(q), scd, i, xs);
+}
+
 // PF: L2 prefetch of the streams ahead of the next group's loads. The single-
 // beam kernel runs faster without it (0.72 against 0.77 ms/step on the
 // 1.28M-node beam), the batch kernel with it (0.897 against 1.020 ms/step on a
@@ -750,8 +850,6 @@ __device__ __forceinline__ void slice_forces_x(const Dev &d, int64_t sl, int lan
     if (i < nN) { ui = urh[i]; li = url[i]; }
     tx = 0.0; ty = 0.0; tz = 0.0;
     double ax = 0.0, ay = 0.0, az = 0.0;
-    const float s0f = (float)d.s0q, guardf = (float)d.guard, scf0 = (float)d.P.sc;
-    const float steelf = (float)d.P.sc_steel;
 
     const int ng = (dg + 3) >> 2;
     Group<CID> Gc, Gn;
@@ -761,56 +859,9 @@ __device__ __forceinline__ void slice_forces_x(const Dev &d, int64_t sl, int lan
         if (PF && g + kPrefetch < ng) prefetch_group<CID, SCE>(d, e0 + 128 * kPrefetch);
         if (g + 1 < ng) load_group<CID>(d, e0 + 128, Gn);
         const int nq = min(4, dg - 4 * g);
-        // padding slots name node 0 and dictionary entry 0 (see slice_forces)
-        float4 uj[4];
-        float2 lj[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t j = group_w(Gc, q) & COL_MASK;
-            uj[q] = urh[j];
-            lj[q] = url[j];
-        }
-        // pass 1: the fast path of all entries of the group, without branches,
-        // so that the four dependency chains interleave
         float fxq[4], fyq[4], fzq[4];
-        unsigned slow = 0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const bool valid = q < nq;
-            const int64_t e = e0 + q;
-            const uint32_t w = group_w(Gc, q), c = Gc.cid(q), sv = (Gc.s >> (8 * q)) & 0xFFu;
-            const int bt = (w >> BT_SHIFT) & 3;
-            float4 A, Bv;
-            ldg_dictx(d.dictx, c, A, Bv);
-            const float etx = (uj[q].x - ui.x) + (uj[q].w - ui.w);
-            const float ety = (uj[q].y - ui.y) + (lj[q].x - li.x);
-            const float etz = (uj[q].z - ui.z) + (lj[q].y - li.y);
-            const float ex = A.x + etx, ey = A.y + ety, ez = A.z + etz;
-            const float L2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
-            const float rL = rsqrtf(L2);
-            const float L = L2 * rL;
-            const float num = __fmaf_rn(etz, A.z + ez, __fmaf_rn(ety, A.y + ey, __fmaf_rn(etx, A.x + ex, Bv.y)));
-            const float sf = __fdividef(num, A.w * (L + A.w));
-            // Fast iff the law is quiet and sf is outside the guard band round
-            // the critical stretch (band edges rounded outwards); a NaN
-            // stretch (zero, infinite or NaN length) fails every comparison.
-            const float scf = has_sce<SCE>(d) ? (float)__ldcs(d.sce + e) : scf0;
-            bool fast;
-            if (LAW == BBPD_LAW_LINEAR) {
-                const float critf = (bt == 0) ? scf : (bt == 1 ? 3.f * scf : steelf);
-                fast = sf <= __fsub_rd(critf, guardf);
-            } else {
-                const float top = (bt == 0) ? s0f : INFINITY;
-                fast = sf <= top && (sf <= __fsub_rd(scf, guardf) || sf >= __fadd_ru(scf, guardf));
-            }
-            fast = fast && sv == 0 && Bv.z != 0.f;
-            const float qf = Bv.x * sf * rL;
-            fxq[q] = qf * ex;
-            fyq[q] = qf * ey;
-            fzq[q] = qf * ez;
-            if (valid && !fast) slow |= 1u << q;
-        }
-        // pass 2: the sum in the reference's order; a full group with no
+        const unsigned slow = group_fast_x<LAW, CID, SCE>(d, Gc, e0, urh, url, ui, li, fxq, fyq, fzq) & ((1u << nq) - 1);
+        // the sum in the reference's order; a full group with no
         // general entry and no chunk start adds its four forces straight
         const uint32_t chunk = (Gc.w.x | Gc.w.y | Gc.w.z | Gc.w.w) & F_CHUNK;
         if (nq == 4 && (slow | chunk) == 0) {
@@ -824,15 +875,9 @@ __device__ __forceinline__ void slice_forces_x(const Dev &d, int64_t sl, int lan
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (q < nq) {
-                const uint32_t w = group_w(Gc, q);
-                double3 r;
-                if (slow & (1u << q)) {
-                    const double scd = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
-                    r = entry_general_x<LAW>(d, e0 + q, w, (Gc.s >> (8 * q)) & 0xFFu, Gc.cid(q), scd, i, xs);
-                } else {
-                    r = make_double3((double)fxq[q], (double)fyq[q], (double)fzq[q]);
-                }
-                if (w & F_CHUNK) {  // partial of the previous OpenMP thread is complete
+                double3 r = make_double3((double)fxq[q], (double)fyq[q], (double)fzq[q]);
+                if (slow & (1u << q)) r = group_slow_x<LAW, CID, SCE>(d, Gc, q, e0, i, xs);
+                if (group_w(Gc, q) & F_CHUNK) {  // partial of the previous OpenMP thread is complete
                     tx = tx + ax; ty = ty + ay; tz = tz + az;
                     ax = 0.0; ay = 0.0; az = 0.0;
                 }
@@ -843,8 +888,6 @@ __device__ __forceinline__ void slice_forces_x(const Dev &d, int64_t sl, int lan
     }
     tx = tx + ax; ty = ty + ay; tz = tz + az;
 }
-
-
 
 // Coordinates for which the shared-divisor division of divide.cuh is exact:
 // +0, or a magnitude in [2^-100, 2^100] (a -0 coordinate could make a -0
@@ -1008,16 +1051,26 @@ __device__ __forceinline__ void ec_integrate_node(const Dev &d, const StepBufs &
     if (far) atomicOr(d.sticky, 1u);
 }
 
+// Sum over the 32 lanes by the xor butterfly (every lane gets it).
+__device__ __forceinline__ void butterfly(double &c1, double &c2, double &c3)
+{
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+        c1 = c1 + __shfl_xor_sync(0xffffffffu, c1, off);
+        c2 = c2 + __shfl_xor_sync(0xffffffffu, c2, off);
+        c3 = c3 + __shfl_xor_sync(0xffffffffu, c3, off);
+    }
+}
+
 // ADR: calculatedampingcoefficient.m:61-85 terms of the nodes of slice sl
 // (lane's node has force tx, ty, tz) and their share of the reaction (force on
-// the prescribed DOFs), folded over the slice's 32 lanes by the xor butterfly
-// and entered into the tree.
-__device__ __forceinline__ void adr_slice_terms(const Dev &d, const StepBufs &b, int64_t sl, int lane,
-                                                double tx, double ty, double tz, int64_t it)
+// the prescribed DOFs), folded over the slice's 32 lanes.
+__device__ __forceinline__ void adr_partial(const Dev &d, const StepBufs &b, int64_t sl, int lane, double tx, double ty,
+                                            double tz, double &c1, double &c2, double &c3)
 {
     const int64_t nN = d.n_nodes;
     const int64_t i = sl * 32 + lane;
-    double c1 = 0, c2 = 0, c3 = 0;
+    c1 = 0; c2 = 0; c3 = 0;
     if (i < nN) {
         const double m = d.mass[i];
         const double Fv[3] = {tx, ty, tz};
@@ -1037,12 +1090,15 @@ __device__ __forceinline__ void adr_slice_terms(const Dev &d, const StepBufs &b,
             c2 = c2 + ue * ue;
         }
     }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) {
-        c1 = c1 + __shfl_xor_sync(0xffffffffu, c1, off);
-        c2 = c2 + __shfl_xor_sync(0xffffffffu, c2, off);
-        c3 = c3 + __shfl_xor_sync(0xffffffffu, c3, off);
-    }
+    butterfly(c1, c2, c3);
+}
+
+// The same entered into the tree.
+__device__ __forceinline__ void adr_slice_terms(const Dev &d, const StepBufs &b, int64_t sl, int lane,
+                                                double tx, double ty, double tz, int64_t it)
+{
+    double c1, c2, c3;
+    adr_partial(d, b, sl, lane, tx, ty, tz, c1, c2, c3);
     tree_publish(d, sl, lane, c1, c2, c3, it);
 }
 
@@ -1067,10 +1123,9 @@ __device__ __forceinline__ void finish_slice(const Dev &d, const StepBufs &b, in
 // ADR phase B (timeintegrationADR.m:53-80) on the nodes of slice sb.
 template <int PREC>
 __device__ __forceinline__ void adr_update_slice(const Dev &d, const StepBufs &b, int64_t sb, int lane,
-                                                 int64_t it)
+                                                 int64_t it, double cn)
 {
     const int64_t nN = d.n_nodes;
-    const double cn = __ldcg(&d.scal[0]);
     {
         const int64_t i = sb * 32 + lane;
         if (i >= nN) return;
@@ -1114,9 +1169,9 @@ __device__ __forceinline__ void adr_update_slice(const Dev &d, const StepBufs &b
 // ADR phase B on slices gwarp, gwarp + nwarps, ...
 template <int PREC>
 __device__ __forceinline__ void adr_update(const Dev &d, const StepBufs &b, int lane, int64_t gwarp,
-                                           int64_t nwarps, int64_t it)
+                                           int64_t nwarps, int64_t it, double cn)
 {
-    for (int64_t sb = gwarp; sb < d.n_slices; sb += nwarps) adr_update_slice<PREC>(d, b, sb, lane, it);
+    for (int64_t sb = gwarp; sb < d.n_slices; sb += nwarps) adr_update_slice<PREC>(d, b, sb, lane, it, cn);
 }
 
 // Global-gather kernel: neighbour data read from HBM/L2 per entry. Used for
@@ -1156,7 +1211,228 @@ __global__ void __launch_bounds__(kBlock, PREC == kP32X ? BBPD_MIN_BLOCKS_F32 : 
         }
         if (SCHEME == BBPD_SCHEME_ADR) {
             if (!bar.wait()) return;
-            adr_update<PREC>(d, b, lane, gwarp, nwarps, it);
+            adr_update<PREC>(d, b, lane, gwarp, nwarps, it, __ldcg(&d.scal[0]));
+        }
+        if (!bar.wait()) return;
+        if (d.n_pen && blockIdx.x == 0 && threadIdx.x == 0) contact_reaction(d, b.n, it);
+    }
+}
+
+// ---------------------------------------------------------------- split kernel
+//
+// step_kernel for problems with too few slices to fill the warps of the GPU: a
+// warp that walks a whole list takes about 31 groups one after the other, so a
+// small beam pays that chain on a few warps while most SMs idle. Here the 8
+// warps of a block share one slice: warp w computes the groups w, w + 8, ... of
+// all 32 lists and leaves their forces in shared memory; then three warps, one
+// per component, add each node's forces in bond order with the OpenMP chunk
+// partials, so every sum keeps the order, and the bits, of step_kernel. The
+// last warp integrates (or enters the ADR tree) while the others start the
+// block's next slice. A block has 16 warps where every slice can have an SM to
+// itself, else 8 and two blocks share an SM, so that one computes while the other
+// sums. What bounds it: the latency of the gathers and of the FP64 chain of two
+// (or four) groups, then 122 dependent additions, then the barriers.
+
+constexpr int kSplitBlock = 512;   // threads of the larger block
+constexpr int kPassGroups = 32;   // groups of 4 entries held in shared memory at a time (128 entries)
+constexpr size_t kSplitSmem = sizeof(double) * 3 * kPassGroups * 4 * 32;
+
+// The slice partials of the Rayleigh-quotient sums folded to cn by one block, in
+// the order of tree_publish. Every block does it for itself after the barrier
+// that follows the partials: with at most kSplitMax slices that is a few KB from
+// L2, and no arrival, fence or further barrier stands in the slices' way.
+constexpr int kSplitMax = 2048;
+constexpr int kSplitGroups = kSplitMax / 32;
+
+__device__ __forceinline__ double block_fold(const Dev &d, int lane, int w, int64_t it)
+{
+    __shared__ double s_sum[3][kSplitGroups];
+    __shared__ double s_cn;
+    int cnt = (int)d.n_slices;
+    const int n2 = (cnt + 31) / 32;
+    for (int g = w; g < n2; g += (int)(blockDim.x >> 5)) {
+        const int k = g * 32 + lane;
+        double2 v = make_double2(0.0, 0.0);
+        double v3 = 0.0;
+        if (k < cnt) {
+            v = __ldcg(&d.tree[k]);
+            v3 = __ldcg(&d.tree3[k]);
+        }
+        if (cnt > 1) butterfly(v.x, v.y, v3);
+        if (lane == 0) {
+            s_sum[0][g] = v.x;
+            s_sum[1][g] = v.y;
+            s_sum[2][g] = v3;
+        }
+    }
+    __syncthreads();
+    if (w == 0) {
+        double c1 = 0.0, c2 = 0.0, c3 = 0.0;   // of the group this lane stands for
+        for (int g = 0; g * 32 < n2; g++) {
+            const int k = g * 32 + lane;
+            double a1 = 0.0, a2 = 0.0, a3 = 0.0;
+            if (k < n2) {
+                a1 = s_sum[0][k];
+                a2 = s_sum[1][k];
+                a3 = s_sum[2][k];
+            }
+            if (n2 > 1) butterfly(a1, a2, a3);
+            if (lane == g) {
+                c1 = a1;
+                c2 = a2;
+                c3 = a3;
+            }
+        }
+        if (n2 > 32) butterfly(c1, c2, c3);
+        if (lane == 0) {
+            const double cn = cn_from_sums(c1, c2);
+            s_cn = cn;
+            if (blockIdx.x == 0) {
+                d.scal[0] = cn;
+                d.scal[1] = c1;
+                d.scal[2] = c2;
+                d.scal[3] = c3;
+                if (it < d.react_cap) d.react[it] = c3;
+            }
+        }
+    }
+    __syncthreads();
+    return s_cn;
+}
+
+template <int LAW, int SCHEME, int PREC, class CID, bool SCE>
+__global__ void __launch_bounds__(kSplitBlock, 1) split_kernel(Dev d, int64_t step0, int64_t nsteps)
+{
+    extern __shared__ double sF[];   // force of entry k of lane l, component c: [(c * 4 kPassGroups + k) * 32 + l]
+    __shared__ double sT[2][3][32];
+    __shared__ uint8_t sC[kPassGroups][32];   // chunk-start bits of a group
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nteam = blockDim.x >> 5;
+    const int64_t gwarp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t nN = d.n_nodes;
+    constexpr int kC = 4 * kPassGroups * 32;
+
+    GridBarrier bar(d.bar, d.err, d.timeout_ns);
+    for (int64_t it = 0; it < nsteps; it++) {
+        const StepBufs b = step_bufs(d, step0 + it);
+        const bool safe = (*(volatile unsigned *)d.sticky & 1u) == 0;
+        if (d.n_pen && blockIdx.x == 0 && threadIdx.x == 0) contact_advance(d, b.n);
+        int par = 0;
+        for (int64_t sl = blockIdx.x; sl < d.n_slices; sl += gridDim.x, par ^= 1) {
+            const int64_t i = sl * 32 + lane;
+            const int dg = (i < nN) ? d.deg[i] : 0;
+            const int64_t sb = d.slice_ptr[sl];
+            const int ngs = d.slice_len[sl] >> 2;
+            double xi = 0, yi = 0, zi = 0;
+            float4 ui = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 li = make_float2(0.f, 0.f);
+            if (i < nN) {
+                if (PREC == kP32X) { ui = b.urhs[i]; li = b.urls[i]; }
+                else { xi = b.xs[i]; yi = b.xs[i + nN]; zi = b.xs[i + 2 * nN]; }
+            }
+            double t = 0.0, a = 0.0;   // warps 0 .. 2: sum of component w of the lane's node
+            for (int G0 = 0; G0 < ngs; G0 += kPassGroups) {
+                const int G1 = min(ngs, G0 + kPassGroups);
+                if (G0 > 0) __syncthreads();   // the previous pass has been added
+                Group<CID> Gc, Gn;
+                int64_t e0 = entry_pos(sb, 4 * (G0 + w), lane);
+                if (G0 + w < G1) load_group<CID>(d, e0, Gc);
+                for (int g = G0 + w; g < G1; g += nteam, e0 += 128 * nteam) {
+                    if (g + nteam < G1) load_group<CID>(d, e0 + 128 * nteam, Gn);
+                    const int nq = max(0, min(4, dg - 4 * g));
+                    double fx[4], fy[4], fz[4];
+                    unsigned slow;
+                    if (PREC == kP32X) {
+                        float gx[4], gy[4], gz[4];
+                        slow = group_fast_x<LAW, CID, SCE>(d, Gc, e0, b.urhs, b.urls, ui, li, gx, gy, gz);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) { fx[q] = (double)gx[q]; fy[q] = (double)gy[q]; fz[q] = (double)gz[q]; }
+                    } else {
+                        slow = group_fast<LAW, CID, SCE>(d, Gc, e0, safe, b.xas, xi, yi, zi, fx, fy, fz);
+                    }
+                    unsigned cb = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        double3 r = make_double3(fx[q], fy[q], fz[q]);
+                        if (q >= nq) {
+                            r = make_double3(-0.0, -0.0, -0.0);   // x + -0 is x, whatever x
+                        } else {
+                            if (slow & (1u << q)) {
+                                if (PREC == kP32X) r = group_slow_x<LAW, CID, SCE>(d, Gc, q, e0, i, b.xs);
+                                else r = group_slow<LAW, PREC, CID, SCE>(d, Gc, q, e0, b.xs, xi, yi, zi);
+                            }
+                            if (group_w(Gc, q) & F_CHUNK) cb |= 1u << q;
+                        }
+                        double *f = sF + (4 * (g - G0) + q) * 32 + lane;
+                        f[0] = r.x;
+                        f[kC] = r.y;
+                        f[2 * kC] = r.z;
+                    }
+                    sC[g - G0][lane] = (uint8_t)cb;
+                    Gc = Gn;
+                }
+                __syncthreads();
+                if (w < 3) {
+                    // 16 values at a time, the next 16 on their way from shared
+                    // memory meanwhile: the chain of additions is what is left
+                    const double *f = sF + w * kC + lane;
+                    const int np = G1 - G0;
+                    auto load16 = [&](int g, double (&v)[16], unsigned &cb) {
+                        cb = 0;
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const bool in = g + q < np;
+                            if (in) cb |= (unsigned)sC[g + q][lane] << (4 * q);
+#pragma unroll
+                            for (int k = 0; k < 4; k++) v[4 * q + k] = in ? f[(4 * (g + q) + k) * 32] : -0.0;
+                        }
+                    };
+                    auto add16 = [&](const double (&v)[16], unsigned cb) {
+                        if (__any_sync(0xffffffffu, cb != 0)) {
+#pragma unroll
+                            for (int k = 0; k < 16; k++) {
+                                if (cb & (1u << k)) {   // partial of the previous OpenMP thread is complete
+                                    t = t + a;
+                                    a = 0.0;
+                                }
+                                a = a + v[k];
+                            }
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 16; k++) a = a + v[k];
+                        }
+                    };
+                    double v0[16], v1[16];
+                    unsigned c0, c1;
+                    load16(0, v0, c0);
+                    for (int g = 0; g < np; g += 8) {
+                        load16(g + 4, v1, c1);
+                        add16(v0, c0);
+                        load16(g + 8, v0, c0);
+                        add16(v1, c1);
+                    }
+                }
+            }
+            if (w < 3) sT[par][w][lane] = t + a;
+            __syncthreads();
+            if (w == nteam - 1) {
+                const double tx = sT[par][0][lane], ty = sT[par][1][lane], tz = sT[par][2][lane];
+                if (SCHEME == BBPD_SCHEME_EULERCROMER) {
+                    if (i < nN) ec_integrate_node<PREC>(d, b, i, tx, ty, tz, it);
+                } else {
+                    if (i < nN) { b.Fc[i] = tx; b.Fc[i + nN] = ty; b.Fc[i + 2 * nN] = tz; }
+                    double c1, c2, c3;
+                    adr_partial(d, b, sl, lane, tx, ty, tz, c1, c2, c3);
+                    if (lane == 0) {
+                        d.tree[sl] = make_double2(c1, c2);
+                        d.tree3[sl] = c3;
+                    }
+                }
+            }
+        }
+        if (SCHEME == BBPD_SCHEME_ADR) {
+            if (!bar.wait()) return;
+            adr_update<PREC>(d, b, lane, gwarp, nwarps, it, block_fold(d, lane, w, it));
         }
         if (!bar.wait()) return;
         if (d.n_pen && blockIdx.x == 0 && threadIdx.x == 0) contact_reaction(d, b.n, it);
@@ -1434,7 +1710,7 @@ __global__ void __launch_bounds__(kBlock, 2) tstep_kernel(Dev d, int64_t step0, 
         }
         if (SCHEME == BBPD_SCHEME_ADR) {
             if (!bar.wait()) return;
-            adr_update<PREC>(d, b, lane, gwarp, nwarps, it);
+            adr_update<PREC>(d, b, lane, gwarp, nwarps, it, __ldcg(&d.scal[0]));
         }
         if (!bar.wait()) return;
         if (d.n_pen && blockIdx.x == 0 && threadIdx.x == 0) contact_reaction(d, b.n, it);
@@ -1648,7 +1924,7 @@ __global__ void __launch_bounds__(kBlock, 2) lstep_kernel(Dev d, int64_t step0, 
                 adr_slice_terms(d, b, sl, lane, fx, fy, fz, it);
             }
             if (!bar.wait()) return;
-            adr_update<kP64>(d, b, lane, gwarp, nwarps, it);
+            adr_update<kP64>(d, b, lane, gwarp, nwarps, it, __ldcg(&d.scal[0]));
         }
         if (!bar.wait()) return;
         if (d.n_pen && blockIdx.x == 0 && threadIdx.x == 0) contact_reaction(d, b.n, it);
@@ -1751,7 +2027,7 @@ __global__ void __launch_bounds__(kBlock, BBPD_MIN_BLOCKS) batch_kernel(BatchCtl
             const int m = member_of(B, w);
             const Dev &d = warp_member(B, m, &s_dev[wib], &s_held[wib], lane);
             const StepBufs b = step_bufs(d, __ldg(&B.mstep[m]) + it);
-            adr_update_slice<PREC>(d, b, w - __ldg(&B.prefix[m]), lane, it);
+            adr_update_slice<PREC>(d, b, w - __ldg(&B.prefix[m]), lane, it, __ldcg(&d.scal[0]));
         }
         if (!bar.wait()) return;
         if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -1830,7 +2106,7 @@ __global__ void __launch_bounds__(kBlock, BBPD_MIN_BLOCKS) batch_kernel_mixed(Ba
             const int m = member_of(B, w);
             const Dev &d = warp_member(B, m, &s_dev[wib], &s_held[wib], lane);
             const StepBufs b = step_bufs(d, __ldg(&B.mstep[m]) + it);
-            adr_update_slice<PREC>(d, b, w - __ldg(&B.prefix[m]), lane, it);
+            adr_update_slice<PREC>(d, b, w - __ldg(&B.prefix[m]), lane, it, __ldcg(&d.scal[0]));
         }
         if (!bar.wait()) return;
         if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -2089,29 +2365,37 @@ __global__ void k_pack_positions(const double *__restrict__ x, int64_t nN, doubl
 typedef void (*kernel_t)(Dev, int64_t, int64_t);
 
 // Instances: law x scheme x precision x dictionary-index width x per-entry
-// critical stretch. Irregular inputs (32-bit dictionary indices) are served
-// with the per-entry critical stretch stream in every case.
+// critical stretch, of step_kernel and split_kernel. Irregular inputs (32-bit
+// dictionary indices) are served with the per-entry critical stretch stream in
+// every case.
+template <int LAW, int SCHEME, int PREC, class CID, bool SCE>
+kernel_t pick_split(bool split)
+{
+    return split ? split_kernel<LAW, SCHEME, PREC, CID, SCE> : step_kernel<LAW, SCHEME, PREC, CID, SCE>;
+}
+
 template <int LAW, int SCHEME, int PREC>
-kernel_t pick_cid(bool wide, bool sce)
+kernel_t pick_cid(bool wide, bool sce, bool split)
 {
     if constexpr (PREC != kP32X) {   // the dictionary-vector form only runs with 16-bit ids
-        if (wide) return step_kernel<LAW, SCHEME, PREC, uint32_t, true>;
+        if (wide) return pick_split<LAW, SCHEME, PREC, uint32_t, true>(split);
     }
-    return sce ? step_kernel<LAW, SCHEME, PREC, uint16_t, true> : step_kernel<LAW, SCHEME, PREC, uint16_t, false>;
+    return sce ? pick_split<LAW, SCHEME, PREC, uint16_t, true>(split)
+               : pick_split<LAW, SCHEME, PREC, uint16_t, false>(split);
 }
 
 template <int LAW, int SCHEME>
-kernel_t pick_prec(int prec, bool wide, bool sce)
+kernel_t pick_prec(int prec, bool wide, bool sce, bool split)
 {
-    if (prec == kP32X) return pick_cid<LAW, SCHEME, kP32X>(wide, sce);
-    return pick_cid<LAW, SCHEME, kP64>(wide, sce);
+    if (prec == kP32X) return pick_cid<LAW, SCHEME, kP32X>(wide, sce, split);
+    return pick_cid<LAW, SCHEME, kP64>(wide, sce, split);
 }
 
 template <int LAW>
-kernel_t pick_scheme(int scheme, int prec, bool wide, bool sce)
+kernel_t pick_scheme(int scheme, int prec, bool wide, bool sce, bool split)
 {
-    return scheme == BBPD_SCHEME_ADR ? pick_prec<LAW, BBPD_SCHEME_ADR>(prec, wide, sce)
-                                     : pick_prec<LAW, BBPD_SCHEME_EULERCROMER>(prec, wide, sce);
+    return scheme == BBPD_SCHEME_ADR ? pick_prec<LAW, BBPD_SCHEME_ADR>(prec, wide, sce, split)
+                                     : pick_prec<LAW, BBPD_SCHEME_EULERCROMER>(prec, wide, sce, split);
 }
 
 template <int LAW, int SCHEME>
@@ -2160,17 +2444,26 @@ lkernel_t pick_lkernel(int law, int scheme, bool sce)
     }
 }
 
-kernel_t pick_kernel(int law, int scheme, int prec, bool wide, bool sce)
+kernel_t pick_kernel(int law, int scheme, int prec, bool wide, bool sce, bool split)
 {
     switch (law) {
-    case BBPD_LAW_LINEAR: return pick_scheme<BBPD_LAW_LINEAR>(scheme, prec, wide, sce);
-    case BBPD_LAW_BILINEAR: return pick_scheme<BBPD_LAW_BILINEAR>(scheme, prec, wide, sce);
-    case BBPD_LAW_TRILINEAR: return pick_scheme<BBPD_LAW_TRILINEAR>(scheme, prec, wide, sce);
-    default: return pick_scheme<BBPD_LAW_EXPONENTIAL>(scheme, prec, wide, sce);
+    case BBPD_LAW_LINEAR: return pick_scheme<BBPD_LAW_LINEAR>(scheme, prec, wide, sce, split);
+    case BBPD_LAW_BILINEAR: return pick_scheme<BBPD_LAW_BILINEAR>(scheme, prec, wide, sce, split);
+    case BBPD_LAW_TRILINEAR: return pick_scheme<BBPD_LAW_TRILINEAR>(scheme, prec, wide, sce, split);
+    default: return pick_scheme<BBPD_LAW_EXPONENTIAL>(scheme, prec, wide, sce, split);
     }
 }
 
 // ------------------------------------------------------------------ host side
+
+// Slices up to which split_kernel runs instead of step_kernel: 6 per SM. Below,
+// a warp a slice leaves most warps without work and the step is one warp's
+// chain; above, every SM has enough warps and the split form's shared-memory
+// round trip costs more than it saves. us per step on B200, step_kernel against
+// split_kernel, ADR: 23 slices 34.8 / 14.7, 203: 41.9 / 19.3, 625: 42.0 / 33.1,
+// 1080: 44.3 / 48.9, 1792: 70.7 / 73.7; Euler-Cromer: 23: 28.8 / 8.7, 203: 32.5 /
+// 12.2, 625: 32.8 / 24.0, 1080: 34.4 / 37.0.
+int64_t split_limit(int nsm) { return std::min<int64_t>(kSplitMax, 6 * (int64_t)nsm); }
 
 unsigned host_threads()
 {
@@ -2397,11 +2690,12 @@ struct bbpd_solver {
     int64_t device_bytes = 0;
     double bytes_per_step = 0;
     kernel_t kernel = nullptr;
-    int grid = 0;
+    int grid = 0, block = kBlock;
     bool tiled = false;                 // tiled kernel with shared-memory staging
     bool lattice = false;               // lattice form (lstep_kernel)
+    bool split = false;                 // a slice per block (split_kernel)
     LTab ltab{};                        // its chain table, a launch argument
-    size_t smem = 0;                    // its dynamic shared memory per block
+    size_t smem = 0;                    // dynamic shared memory per block
     bbpd_batch *batch = nullptr;        // batch this solver is a member of
     bool has_density = false;          // DENSITY given (contact needs it)
     bool cn_stale = false;              // cn on the device is newer than S->cn
@@ -3682,6 +3976,10 @@ extern "C" int bbpd_create(const bbpd_problem *pb, const bbpd_params *prm, int d
         for (int64_t k = 0; k < nB; k++) m = std::fmin(m, pb->s0[k]);
         d.s0q = m;
     }
+    // the softening laws act above s0; the brittle law above the least of the
+    // three critical stretches of calculatebondfailureMex.c:36-38
+    d.quiet_hi = quiet_high_word(d.s0q);
+    if (prm->law == BBPD_LAW_LINEAR) d.quiet_hi = quiet_high_word(std::fmin(prm->sc, std::fmin(3 * prm->sc, prm->sc_steel)));
     P.beta = prm->beta_tri;
     double eta = prm->s1 / prm->s0;
     P.tri_c1 = (eta - P.beta) / (eta - 1);
@@ -3703,6 +4001,8 @@ extern "C" int bbpd_create(const bbpd_problem *pb, const bbpd_params *prm, int d
     d.timeout_ns = (unsigned long long)(to * 1e9);
 
     // kernel and grid
+    int nsm = 0, occ = 0, coop = 0;
+    BBPD_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     if (S->lattice) {
         S->kernel = reinterpret_cast<kernel_t>(pick_lkernel(prm->law, prm->scheme, pb->sc != nullptr));
         BBPD_CUDA_TRY(cudaFuncSetAttribute((const void *)S->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3712,15 +4012,21 @@ extern "C" int bbpd_create(const bbpd_problem *pb, const bbpd_params *prm, int d
         BBPD_CUDA_TRY(cudaFuncSetAttribute((const void *)S->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)S->smem));
     } else {
-        S->kernel = pick_kernel(prm->law, prm->scheme, S->prec, S->wide, pb->sc != nullptr);
+        S->split = ns <= split_limit(nsm);
+        S->kernel = pick_kernel(prm->law, prm->scheme, S->prec, S->wide, pb->sc != nullptr, S->split);
+        if (S->split) {
+            S->smem = kSplitSmem;
+            if (ns <= nsm) S->block = kSplitBlock;
+            BBPD_CUDA_TRY(cudaFuncSetAttribute((const void *)S->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)S->smem));
+        }
     }
-    int nsm = 0, occ = 0, coop = 0;
-    BBPD_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     BBPD_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
     if (!coop) return fail(BBPD_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)S->kernel, kBlock, S->smem));
+    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)S->kernel, S->block, S->smem));
     if (occ < 1) return fail(BBPD_ERR_CUDA, "kernel cannot be resident");
-    int64_t want = (ns * 32 + kBlock - 1) / kBlock;   // one warp per slice at most
+    // one warp per slice at most; a block per slice in the split kernel
+    int64_t want = S->split ? ns : (ns * 32 + kBlock - 1) / kBlock;
     S->grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * occ, want));
     BBPD_CUDA_TRY(cudaEventCreate(&S->ev0));
     BBPD_CUDA_TRY(cudaEventCreate(&S->ev1));
@@ -3771,7 +4077,7 @@ extern "C" int bbpd_step_async(bbpd_solver *S, int64_t nsteps)
     void *args[] = {(void *)&S->d, (void *)&step0, (void *)&nsteps, (void *)&S->ltab};   // lattice kernels take the table
     BBPD_CUDA_TRY(cudaMemsetAsync(S->d.work, 0, 2 * sizeof(unsigned long long), S->stream));
     BBPD_CUDA_TRY(cudaEventRecord(S->ev0, S->stream));
-    BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)S->kernel, dim3(S->grid), dim3(kBlock), args, S->smem, S->stream));
+    BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)S->kernel, dim3(S->grid), dim3(S->block), args, S->smem, S->stream));
     BBPD_CUDA_TRY(cudaEventRecord(S->ev1, S->stream));
     S->step += nsteps;
     return BBPD_OK;
@@ -4095,7 +4401,7 @@ extern "C" int bbpd_get_info(bbpd_solver *S, bbpd_info *info)
     info->n_entries = S->ne;
     info->n_slices = S->ns;
     info->grid_blocks = S->grid;
-    info->block_threads = kBlock;
+    info->block_threads = S->block;
     info->device_bytes = S->device_bytes;
     info->bytes_per_step = S->bytes_per_step;
     info->layout = (S->wide ? 2 : (S->prec == kP32X ? 3 : 1)) + (S->tiled ? 16 : 0) + (S->lattice ? 32 : 0);

@@ -494,6 +494,30 @@ def test_lattice_vs_oracle(small, law, scheme):
     s.close()
 
 
+# (nx, ny, nz, horizon factor): one slice; slices on both sides of one per SM
+# (16- and 8-warp blocks); lists longer than the 128 entries a block holds at a
+# time, with a ragged last slice; both sides of the line to step_kernel (6 per SM)
+@pytest.mark.parametrize("nx,ny,nz,hf", [(7, 2, 2, 3.015), (37, 8, 16, 3.015), (53, 10, 9, 3.015),
+                                         (19, 9, 11, 4.1), (37, 24, 32, 3.015), (31, 30, 31, 3.015)])
+@pytest.mark.parametrize("law,scheme", [("trilinear", "adr"), ("linear", "eulercromer"), ("exponential", "adr"),
+                                        ("bilinear", "eulercromer")])
+def test_split_and_step_kernels_vs_oracle(nx, ny, nz, hf, law, scheme):
+    """Bit-identical at the sizes where the kernel or its block changes."""
+    inp = bb.beam.build(bb.beam.small(nx=nx, ny=ny, nz=nz, horizon_factor=hf))
+    kw = dict(LAWKW[law], scheme=scheme, rate=-4e-6)
+    s = bb.Solver(inp, **kw)
+    r = orun(inp, **kw)
+    for n in (1, 14):
+        s.step(n)
+        r.step(n)
+        compare(s, r, law)
+    if scheme == "adr":   # the reaction and the damping coefficient come from the block's own fold
+        assert s.cn == r.cn
+        pf = inp["BODYFORCEFLAG"] == 1
+        np.testing.assert_allclose(s.reaction(14)[13], s.get("force")[pf].sum(), rtol=1e-9, atol=1e-12)
+    s.close()
+
+
 @pytest.fixture(scope="module")
 def ragged():
     """70 x 9 x 11 nodes: partial tiles along every axis (x rows of 32, rows of
