@@ -42,6 +42,7 @@
 // the kernel returns early (status BBPD_ERR_TIMEOUT), never hanging.
 #include "bbpd_internal.h"
 #include "divide.cuh"
+#include "gridbarrier.cuh"
 #include "physics.cuh"
 #include "staging.cuh"
 
@@ -77,8 +78,7 @@ constexpr int LST_BT_SHIFT = 3;          // lattice form: bits 3-4 of the state 
 constexpr uint8_t LST_ABSENT = 0x80;     // lattice form: no bond in this slot
 constexpr int64_t MAX_NODES = (int64_t)1 << 24;
 
-constexpr int ERR_TIMEOUT = 1;
-constexpr int ERR_NONFINITE = 2;
+constexpr int ERR_NONFINITE = 2;   // beside ERR_TIMEOUT (gridbarrier.cuh)
 
 constexpr int kBlock = 256;
 #ifndef BBPD_MIN_BLOCKS
@@ -206,13 +206,6 @@ struct LTab {
     int4 e[kMaxSigma];   // (partner offset in the staged box, slot row base, lower-node offset, 0)
 };
 
-__device__ __forceinline__ unsigned long long globaltimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ double prescribed_value(const Dev &d, int64_t n)
 {
     if (d.amplitude == BBPD_AMP_SMOOTHSTEP) {
@@ -222,30 +215,6 @@ __device__ __forceinline__ double prescribed_value(const Dev &d, int64_t n)
         return v0 + (v1 - v0) * ((xi * xi) * xi) * (10 - 15 * xi + 6 * (xi * xi));
     }
     return d.rate * (double)n;
-}
-
-// Wait until the counter *word has reached `target` (modulo 2^32), at most
-// timeout_ns. Gives up early when another block already reported a timeout in
-// *err. On expiry sets ERR_TIMEOUT in *err and returns false; never waits
-// without a limit. The clock and *err are looked at once in 64 polls, so a poll
-// costs one L2 round trip.
-__device__ bool bounded_wait_reach(const unsigned *word, unsigned target, int *err, unsigned long long timeout_ns)
-{
-    unsigned long long t0 = 0;
-    for (unsigned k = 1;; k++) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-        if ((int)(v - target) >= 0) return true;
-        if ((k & 63u) == 0) {
-            if (*(volatile int *)err & ERR_TIMEOUT) return false;
-            const unsigned long long now = globaltimer();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > timeout_ns) {
-                atomicOr(err, ERR_TIMEOUT);
-                return false;
-            }
-        }
-    }
 }
 
 // Clamp of calculatedampingcoefficient.m:90-112 applied to the two sums.
@@ -338,35 +307,6 @@ __device__ __forceinline__ int64_t grab_counter(unsigned long long *ctr, int lan
 }
 
 __device__ __forceinline__ int64_t grab_slice(const Dev &d, int lane) { return grab_counter(d.work, lane); }
-
-// Grid-wide barrier with a time limit. Arrivals only count up from zero at the
-// launch (the host clears the counter before it), so block and barrier number
-// give the value to wait for: one release addition whose result nobody waits
-// for, then one poll after another, with no generation to read first and none
-// to write at the end. On the 1.28M-node beam's grid of 296 blocks a barrier
-// went from 3 us to 1.3 us.
-struct GridBarrier {
-    unsigned *ctr;
-    unsigned target;
-    int *err;
-    unsigned long long timeout_ns;
-
-    __device__ __forceinline__ GridBarrier(unsigned *c, int *e, unsigned long long t)
-        : ctr(c), target(0), err(e), timeout_ns(t) {}
-    // false when a wait ran out (ERR_TIMEOUT set in *err)
-    __device__ __forceinline__ bool wait()
-    {
-        __shared__ int s_ok;
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
-            s_ok = bounded_wait_reach(ctr, target, err, timeout_ns);
-        }
-        __syncthreads();
-        return s_ok != 0;
-    }
-};
 
 // L2 prefetch of one line: no register is written, so a warp can keep many
 // groups of its streams in flight ahead of the loads that consume them.

@@ -24,10 +24,14 @@
 //
 // Layout: per bond its end nodes, constants and state; per node the list of
 // its bond ends in bond order (a stable radix sort of the directed entries by
-// node), which gives the nodal sums their serial order and the matrix-free
-// products their neighbours. Reductions are two-level and fixed-order, so a
-// step is deterministic.
+// node), which gives the nodal sums their serial order. For the matrix-free
+// products the lists are also laid out in slices of 32 nodes, entry k of the
+// slice's 32 lists side by side (padded to its longest list): the neighbour's id
+// and, per tangent, the bond's stiffness scale, 12 bytes an entry. The bond
+// vector is the difference of the two nodes' positions, which lie in one record
+// with the direction p. Reductions are fixed-order, so a step is deterministic.
 #include "bbpd_internal.h"
+#include "gridbarrier.cuh"
 #include "physics.cuh"
 #include "staging.cuh"
 
@@ -71,7 +75,6 @@ struct SBonds {
     double *fail, *bsf;
     uint8_t *flag;
     double *rig;                // tangent scale, 0 for failed bonds
-    double *c;                  // current bond vector x_b - x_a, [3 nB]
     double *f;                  // bond force, [3 nB]
     int64_t nB;
     int law;
@@ -114,7 +117,6 @@ __global__ void k_static_bonds(SBonds s, const double *__restrict__ x, int64_t n
             double f = t * (d[c] / L);
             if (f != f) f = 0.0;
             s.f[k + c * s.nB] = f;
-            s.c[k + c * s.nB] = d[c];
         }
         // rig = BFM * ((BS / L^3) * VCF * V^2) * (1 - BSF) for intact bonds
         const double r = fl == 1 ? s.BFM[k] * ((s.BS[k] / (L * L * L)) * s.VCF[k] * (s.V * s.V)) * (1 - B) : 0.0;
@@ -125,6 +127,10 @@ __global__ void k_static_bonds(SBonds s, const double *__restrict__ x, int64_t n
 struct SNodes {
     const int64_t *off;         // [n + 1] list offsets
     const uint32_t *ent;        // directed entries q = 2k + side, by node, in bond order
+    const uint32_t *a, *b;      // end nodes of the bonds
+    const int64_t *sptr;        // slots of slice s: [sptr[s], sptr[s + 1])
+    const uint32_t *bond, *col; // bond and neighbour of every slot
+    int64_t ns;
     const uint8_t *held;        // per DOF [3 n]: 1 support, 2 prescribed
     int64_t n, nB;
 };
@@ -174,73 +180,121 @@ __global__ void k_static_nodal(SNodes g, const double *__restrict__ f, double V,
     }
 }
 
-// y = K p on the free DOFs (held DOFs: y = 0, p taken as 0), and a partial of
-// p.y. One warp per node: the lanes take its entries 32 apart and the sums
-// meet in a fixed butterfly, so the product is deterministic.
-__global__ void k_static_spmv(SNodes g, const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
-                              const double *__restrict__ rig, const double *__restrict__ cv,
-                              const double *__restrict__ p, double *y, double *part)
+// The slices: length of each (its longest list), times 32 for the scan
+__global__ void k_slice_lengths(const int64_t *__restrict__ off, int64_t n, int64_t ns, int64_t *cnt)
 {
-    __shared__ double sh[kThreads / 32];
     const int lane = threadIdx.x & 31;
-    double acc = 0;
-    const int64_t n = g.n, nB = g.nB;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        double pi[3];
-        for (int c = 0; c < 3; c++) pi[c] = g.held[i + c * n] ? 0.0 : p[i + c * n];
-        double yi[3] = {0, 0, 0};
-        for (int64_t e = g.off[i] + lane; e < g.off[i + 1]; e += 32) {
-            const uint32_t q = g.ent[e];
-            const int64_t k = q >> 1;
-            const double r = rig[k];
-            if (r == 0) continue;
-            const int64_t j = (q & 1u) ? a[k] : b[k];
-            const double c0 = cv[k], c1 = cv[k + nB], c2 = cv[k + 2 * nB];
-            double dp[3];
-            for (int c = 0; c < 3; c++) dp[c] = pi[c] - (g.held[j + c * n] ? 0.0 : p[j + c * n]);
-            const double t = r * (c0 * dp[0] + c1 * dp[1] + c2 * dp[2]);
-            yi[0] += t * c0;
-            yi[1] += t * c1;
-            yi[2] += t * c2;
-        }
-        for (int o = 16; o > 0; o >>= 1)
-            for (int c = 0; c < 3; c++) yi[c] += __shfl_xor_sync(0xffffffffu, yi[c], o);
-        if (lane == 0)
-            for (int c = 0; c < 3; c++) {
-                const double v = g.held[i + c * n] ? 0.0 : yi[c];
-                y[i + c * n] = v;
-                acc += pi[c] * v;
-            }
-    }
-    if (lane == 0) sh[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0;
-        for (int w = 0; w < kThreads / 32; w++) s += sh[w];
-        part[blockIdx.x] = s;
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s <= ns; s += warps) {
+        const int64_t i = s * 32 + lane;
+        int len = s < ns && i < n ? (int)(off[i + 1] - off[i]) : 0;
+        for (int o = 16; o > 0; o >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
+        if (lane == 0) cnt[s] = (int64_t)len * 32;
     }
 }
 
-// Block-Jacobi preconditioner: the inverse of each node's 3 x 3 diagonal block
-// restricted to its free DOFs (symmetric, 6 values); a DOF without stiffness
-// (every bond of its node broken) is left out of the solve.
-__global__ void k_static_precond(SNodes g, const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
-                                 const double *__restrict__ rig, const double *__restrict__ cv, double *Minv,
-                                 uint8_t *skip)
+constexpr uint32_t kNoBond = 0xFFFFFFFFu;
+
+// Bond and neighbour of every slot; padding names the node itself and no bond
+__global__ void k_slice_fill(const int64_t *__restrict__ off, const uint32_t *__restrict__ ent,
+                             const uint32_t *__restrict__ a, const uint32_t *__restrict__ b, int64_t n, int64_t ns,
+                             const int64_t *__restrict__ sptr, uint32_t *bond, uint32_t *col)
 {
-    const int64_t n = g.n, nB = g.nB;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < ns; s += warps) {
+        const int64_t i = s * 32 + lane, e0 = i < n ? off[i] : 0, e1 = i < n ? off[i + 1] : 0;
+        const int64_t len = (sptr[s + 1] - sptr[s]) >> 5;
+        for (int64_t k = 0; k < len; k++) {
+            const int64_t at = sptr[s] + k * 32 + lane;
+            uint32_t q = kNoBond, j = i < n ? (uint32_t)i : 0u;
+            if (e0 + k < e1) {
+                const uint32_t v = ent[e0 + k];
+                q = v >> 1;
+                j = (v & 1u) ? a[q] : b[q];
+            }
+            bond[at] = q;
+            col[at] = j;
+        }
+    }
+}
+
+// Segments of every slice: warp w sums rows [w chunk, (w + 1) chunk), and its
+// part of slice s is segment s + w
+__global__ void k_segments(const int64_t *__restrict__ sptr, int64_t ns, int64_t chunk, int32_t *seg)
+{
+    GRID_STRIDE(s, ns)
+    {
+        const int64_t a = sptr[s] >> 5, b = sptr[s + 1] >> 5;
+        seg[2 * s] = (int32_t)(s + a / chunk);
+        seg[2 * s + 1] = b > a ? (int32_t)(s + (b - 1) / chunk + 1) : seg[2 * s];
+    }
+}
+
+// A node's position and its component of the CG direction p (zero on held and
+// left-out DOFs): 64 bytes, read as a 256-bit and a 128-bit load
+struct __align__(64) NodeRec {
+    double x, y, z, px, py, pz, pad[2];
+};
+struct Rec6 {
+    double x, y, z, px, py, pz;
+};
+
+__device__ __forceinline__ Rec6 load_rec(const NodeRec *p)
+{
+    Rec6 r;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.px) : "l"(p));
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.py), "=d"(r.pz) : "l"(&p->py));
+    return r;
+}
+
+// What a linear solve reads: position records, every slot's stiffness scale,
+// and the block-Jacobi preconditioner: the inverse of each node's 3 x 3
+// diagonal block restricted to its free DOFs (symmetric, 6 values); a DOF
+// without stiffness (every bond of its node broken) is left out of the solve.
+__global__ void k_static_records(const double *__restrict__ x, int64_t n, NodeRec *rec)
+{
     GRID_STRIDE(i, n)
     {
-        double D[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int64_t e = g.off[i]; e < g.off[i + 1]; e++) {
-            const int64_t k = g.ent[e] >> 1;
-            const double r = rig[k];
+        rec[i].x = x[i];
+        rec[i].y = x[i + n];
+        rec[i].z = x[i + 2 * n];
+    }
+}
+
+__global__ void k_slot_rig(const uint32_t *__restrict__ bond, const double *__restrict__ rig,
+                           const int64_t *__restrict__ slots, double *rigE)
+{
+    GRID_STRIDE(e, *slots)
+    {
+        const uint32_t q = bond[e];
+        rigE[e] = q == kNoBond ? 0.0 : rig[q];
+    }
+}
+
+__global__ void k_static_precond(SNodes g, const double *__restrict__ rig, const NodeRec *__restrict__ rec, double *Minv,
+                                 uint8_t *skip)
+{
+    const int64_t n = g.n;
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const double xi[3] = {rec[i].x, rec[i].y, rec[i].z};
+        double S[6] = {0, 0, 0, 0, 0, 0};   // D00 D01 D02 D11 D12 D22
+        for (int64_t e = g.off[i] + lane; e < g.off[i + 1]; e += 32) {
+            const uint32_t q = g.ent[e];
+            const double r = rig[q >> 1];
             if (r == 0) continue;
-            const double c[3] = {cv[k], cv[k + nB], cv[k + 2 * nB]};
+            const NodeRec *o = rec + ((q & 1u) ? g.a[q >> 1] : g.b[q >> 1]);
+            const double c[3] = {o->x - xi[0], o->y - xi[1], o->z - xi[2]};
+            int k = 0;
             for (int u = 0; u < 3; u++)
-                for (int v = 0; v < 3; v++) D[u][v] += r * c[u] * c[v];
+                for (int v = u; v < 3; v++) S[k++] += r * c[u] * c[v];
         }
+        for (int o = 16; o > 0; o >>= 1)
+            for (int q = 0; q < 6; q++) S[q] += __shfl_xor_sync(0xffffffffu, S[q], o);
+        if (lane != 0) continue;
+        double D[3][3] = {{S[0], S[1], S[2]}, {S[1], S[3], S[4]}, {S[2], S[4], S[5]}};
         bool fr[3];
         for (int u = 0; u < 3; u++) {
             fr[u] = !g.held[i + u * n] && D[u][u] > 0;
@@ -273,131 +327,278 @@ __global__ void k_static_precond(SNodes g, const uint32_t *__restrict__ a, const
     }
 }
 
-__device__ __forceinline__ void apply_minv(const double *Minv, int64_t i, int64_t n, const double r[3], double z[3])
+__device__ __forceinline__ void apply_minv(const double m[6], const double r[3], double z[3])
 {
-    const double m0 = Minv[i], m1 = Minv[i + n], m2 = Minv[i + 2 * n], m3 = Minv[i + 3 * n], m4 = Minv[i + 4 * n],
-                 m5 = Minv[i + 5 * n];
-    z[0] = m0 * r[0] + m1 * r[1] + m2 * r[2];
-    z[1] = m1 * r[0] + m3 * r[1] + m4 * r[2];
-    z[2] = m2 * r[0] + m4 * r[1] + m5 * r[2];
+    z[0] = m[0] * r[0] + m[1] * r[1] + m[2] * r[2];
+    z[1] = m[1] * r[0] + m[3] * r[1] + m[4] * r[2];
+    z[2] = m[2] * r[0] + m[4] * r[1] + m[5] * r[2];
 }
 
-// CG start: delta = 0, r = F on the solved DOFs, z = M^-1 r, p = z; partials
-// of r.z and r.r
-__global__ void k_cg_init(int64_t n, const double *__restrict__ F, const uint8_t *__restrict__ skip,
-                          const double *__restrict__ Minv, double *d, double *r, double *z, double *p, double *part)
-{
-    __shared__ double sh[2][kThreads / 32];
-    double rz = 0, rr = 0;
-    GRID_STRIDE(i, n)
-    {
-        double ri[3], zi[3];
-        for (int c = 0; c < 3; c++) ri[c] = skip[i + c * n] ? 0.0 : F[i + c * n];
-        apply_minv(Minv, i, n, ri, zi);
-        for (int c = 0; c < 3; c++) {
-            if (skip[i + c * n]) zi[c] = 0.0;
-            d[i + c * n] = 0.0;
-            r[i + c * n] = ri[c];
-            z[i + c * n] = zi[c];
-            p[i + c * n] = zi[c];
-            rz += ri[c] * zi[c];
-            rr += ri[c] * ri[c];
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        rz += __shfl_xor_sync(0xffffffffu, rz, o);
-        rr += __shfl_xor_sync(0xffffffffu, rr, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][threadIdx.x >> 5] = rz;
-        sh[1][threadIdx.x >> 5] = rr;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s0 = 0, s1 = 0;
-        for (int w = 0; w < kThreads / 32; w++) {
-            s0 += sh[0][w];
-            s1 += sh[1][w];
-        }
-        part[2 * blockIdx.x] = s0;
-        part[2 * blockIdx.x + 1] = s1;
-    }
-}
-
-// Sum of `w` interleaved partial streams of `nb` blocks, in block order, to out[0..w)
+// Sum of `w` interleaved partial streams of `nb` blocks to out[0..w): one warp
+// per stream, lanes 32 apart, then the butterfly
 __global__ void k_reduce(const double *__restrict__ part, int nb, int w, double *out)
 {
-    if (threadIdx.x < w) {
-        double s = 0;
-        for (int b = 0; b < nb; b++) s += part[b * w + threadIdx.x];
-        out[threadIdx.x] = s;
-    }
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (k >= w) return;
+    double s = 0;
+    for (int b = lane; b < nb; b += 32) s += part[b * w + k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[k] = s;
 }
 
-// scal: [0] r.z, [1] r.r, [2] p.Kp, [3] alpha
-// delta += alpha p, r -= alpha Kp, z = M^-1 r; partials of the new r.z, r.r
-__global__ void k_cg_update(int64_t n, const uint8_t *__restrict__ skip, const double *__restrict__ Minv,
-                            const double *__restrict__ scal, const double *__restrict__ p,
-                            const double *__restrict__ Kp, double *d, double *r, double *z, double *part)
+// Two sums over the block's threads, in a fixed order (every thread gets them)
+__device__ __forceinline__ void block_sum2(double &u, double &v, double (*sh)[32])
 {
-    __shared__ double sh[2][kThreads / 32];
-    const double alpha = scal[2] != 0 ? scal[0] / scal[2] : 0.0;
-    double rz = 0, rr = 0;
-    GRID_STRIDE(i, n)
-    {
-        double ri[3], zi[3];
-        for (int c = 0; c < 3; c++) {
-            const int64_t e = i + c * n;
-            d[e] += alpha * p[e];
-            ri[c] = r[e] - alpha * Kp[e];
-            if (skip[e]) ri[c] = 0.0;
-            r[e] = ri[c];
-        }
-        apply_minv(Minv, i, n, ri, zi);
-        for (int c = 0; c < 3; c++) {
-            if (skip[i + c * n]) zi[c] = 0.0;
-            z[i + c * n] = zi[c];
-            rz += ri[c] * zi[c];
-            rr += ri[c] * ri[c];
-        }
-    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int o = 16; o > 0; o >>= 1) {
-        rz += __shfl_xor_sync(0xffffffffu, rz, o);
-        rr += __shfl_xor_sync(0xffffffffu, rr, o);
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+        v += __shfl_xor_sync(0xffffffffu, v, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][threadIdx.x >> 5] = rz;
-        sh[1][threadIdx.x >> 5] = rr;
+    __syncthreads();   // sh is free
+    if (lane == 0) {
+        sh[0][w] = u;
+        sh[1][w] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double s0 = 0, s1 = 0;
-        for (int w = 0; w < kThreads / 32; w++) {
-            s0 += sh[0][w];
-            s1 += sh[1][w];
+    u = lane < nw ? sh[0][lane] : 0.0;
+    v = lane < nw ? sh[1][lane] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) {
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+}
+
+// The grid's two sums: every block publishes its own and, after the barrier,
+// adds all of them for itself in the same order.
+__device__ __forceinline__ bool grid_sum2(double &u, double &v, double (*sh)[32], double2 *part, GridBarrier &bar)
+{
+    block_sum2(u, v, sh);
+    if (threadIdx.x == 0) part[blockIdx.x] = make_double2(u, v);
+    if (!bar.wait()) return false;
+    u = v = 0;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+        const double2 p = __ldcg(&part[k]);
+        u += p.x;
+        v += p.y;
+    }
+    block_sum2(u, v, sh);
+    return true;
+}
+
+constexpr int kCgThreads = 512;   // 16 warps of 128 registers on every SM
+constexpr int kCgRows = 4;         // rows of a warp's gathers in flight
+constexpr int kCgCheck = 8;        // iterations between convergence checks
+constexpr int kCgLaunch = 1024;    // iterations of one launch at most
+
+struct CgArgs {
+    SNodes g;
+    const double *rigE;            // stiffness scale of every slot (0: failed bond or padding)
+    NodeRec *rec;
+    const double *F, *Minv;
+    const uint8_t *skip;
+    double *x;                     // moved by the solution once the solve ends
+    double *d, *r, *z;
+    double *yseg;                  // partial K p of every segment: [segment][component][lane]
+    const int32_t *seg;            // segments of slice s: [seg[2 s], seg[2 s + 1])
+    double2 *part;                 // 2 x gridDim block partials
+    double *scal;                  // [0] r.z, [1] r.r, [2] r.r at the start
+    int *state;                    // [0] CG_*, [1] iterations so far, [2] error word
+    unsigned *bar;
+    unsigned long long timeout_ns;
+    double tol2;                   // stop at r.r <= tol2 * r.r at the start
+    int first, max_cg;
+    int64_t rows;                  // rows of 32 slots, all slices together
+    int64_t chunk;                 // consecutive rows of one warp
+};
+enum { CG_MORE = 0, CG_DONE = 1, CG_NONFINITE = 2 };
+
+// The linear solve K delta = F on the free DOFs by conjugate gradients, one
+// persistent launch: three barriers an iteration (after p.Kp, after r.z and
+// r.r, after the new p) instead of six kernels, two of which summed 592 partials
+// with one thread. In K p a lane stands for a node, so that a warp's 32
+// neighbours lie side by side as the nodes do. Every warp takes the same number
+// of consecutive rows (entry k of a slice's 32 lists), wherever slices begin, and
+// leaves a partial sum per slice it touched (a segment); the update adds the
+// segments of a slice in order. So the warps are equally loaded at every size,
+// and p.Kp needs no complete sums. What bounds it: at 20 000 nodes the latency of
+// 17 rows of gathers and three barriers, at millions the L1 wavefronts of the
+// gathers and 12 bytes an entry. 20 000 nodes, 1.0M bonds, B200: 109 us an
+// iteration with six kernels, 22 here (10 of them barriers, sums and updates);
+// 128 000 nodes 324 and 88. One block of 16 warps per SM ran faster than two at
+// 64 registers (27 us: spills, twice the arrivals).
+__global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
+{
+    __shared__ double sh[2][32];
+    GridBarrier bar(A.bar, A.state + 2, A.timeout_ns);
+    const int64_t n = A.g.n;
+    const int lane = threadIdx.x & 31;
+    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    const int64_t r0 = gw * A.chunk, r1 = min(A.rows, r0 + A.chunk);
+    int64_t sfirst = 0;   // slice of row r0
+    if (r0 < r1)
+        for (int64_t lo = 0, hi = A.g.ns; hi - lo > 1;) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (A.g.sptr[mid] <= r0 * 32) lo = mid;
+            else hi = mid;
+            sfirst = lo;
         }
-        part[2 * blockIdx.x] = s0;
-        part[2 * blockIdx.x + 1] = s1;
+    double2 *part0 = A.part, *part1 = A.part + gridDim.x;
+    double rz, rr, rr0;
+    int done = 0;
+    if (A.first) {
+        // delta = 0, r = F on the solved DOFs, z = M^-1 r, p = z
+        rz = rr = 0;
+        GRID_STRIDE(i, n)
+        {
+            double ri[3], zi[3];
+            for (int c = 0; c < 3; c++) ri[c] = A.skip[i + c * n] ? 0.0 : A.F[i + c * n];
+            double m[6];
+            for (int c = 0; c < 6; c++) m[c] = A.Minv[i + c * n];
+            apply_minv(m, ri, zi);
+            for (int c = 0; c < 3; c++) {
+                if (A.skip[i + c * n]) zi[c] = 0.0;
+                A.d[i + c * n] = 0.0;
+                A.r[i + c * n] = ri[c];
+                rz += ri[c] * zi[c];
+                rr += ri[c] * ri[c];
+            }
+            A.rec[i].px = zi[0];
+            A.rec[i].py = zi[1];
+            A.rec[i].pz = zi[2];
+        }
+        if (!grid_sum2(rz, rr, sh, part0, bar)) return;
+        rr0 = rr;
+    } else {
+        rz = A.scal[0];
+        rr = A.scal[1];
+        rr0 = A.scal[2];
+        done = A.state[1];
+    }
+    int state = rr0 > 0 ? CG_MORE : CG_DONE;   // a NaN r.r has nothing to solve either
+    for (int it = 0; it < kCgLaunch && state == CG_MORE; it++) {
+        // y = K p, p.y
+        double py = 0, unused = 0;
+        for (int64_t row = r0, s = sfirst; row < r1; s++) {
+            const int64_t end = min(r1, A.g.sptr[s + 1] >> 5), i = s * 32 + lane;
+            if (end <= row) continue;   // a slice without bonds
+            Rec6 o = {0, 0, 0, 0, 0, 0};
+            if (i < n) o = load_rec(A.rec + i);
+            double y0 = 0, y1 = 0, y2 = 0;
+            auto add = [&](const Rec6 &q, double r) {
+                const double c0 = q.x - o.x, c1 = q.y - o.y, c2 = q.z - o.z;
+                const double t = r * (c0 * (o.px - q.px) + c1 * (o.py - q.py) + c2 * (o.pz - q.pz));
+                // a failed bond (r = 0) adds nothing, whatever its ends hold
+                y0 += r != 0 ? t * c0 : 0.0;
+                y1 += r != 0 ? t * c1 : 0.0;
+                y2 += r != 0 ? t * c2 : 0.0;
+            };
+            // kCgRows rows at a time, the next rows' streams on their way;
+            // rows past the end repeat the last one with scale 0
+            const uint32_t *col = A.g.col + row * 32 + lane;
+            const double *rig = A.rigE + row * 32 + lane;
+            const int rows = (int)(end - row);
+            uint32_t j[kCgRows];
+            double g[kCgRows];
+            auto streams = [&](int k) {
+#pragma unroll
+                for (int q = 0; q < kCgRows; q++) {
+                    const int at = min(k + q, rows - 1) * 32;
+                    j[q] = __ldg(col + at);
+                    g[q] = k + q < rows ? __ldg(rig + at) : 0.0;
+                }
+            };
+            streams(0);
+            for (int k = 0; k < rows; k += kCgRows) {
+                Rec6 v[kCgRows];
+                double h[kCgRows];
+#pragma unroll
+                for (int q = 0; q < kCgRows; q++) {
+                    v[q] = load_rec(A.rec + j[q]);
+                    h[q] = g[q];
+                }
+                if (k + kCgRows < rows) streams(k + kCgRows);
+#pragma unroll
+                for (int q = 0; q < kCgRows; q++) add(v[q], h[q]);
+            }
+            row = end;
+            double *ys = A.yseg + (s + gw) * 96 + lane;
+            ys[0] = y0;
+            ys[32] = y1;
+            ys[64] = y2;
+            py += o.px * y0 + o.py * y1 + o.pz * y2;   // p is zero on held DOFs
+        }
+        if (!grid_sum2(py, unused, sh, part1, bar)) return;
+        // delta += alpha p, r -= alpha y, z = M^-1 r
+        const double alpha = py != 0 ? rz / py : 0.0;
+        double rzn = 0, rrn = 0;
+        GRID_STRIDE(i, n)
+        {
+            // every load first, then the segments four at a time: one round
+            // trip to L2 for nearly all nodes
+            const int2 q2 = *reinterpret_cast<const int2 *>(A.seg + 2 * (i >> 5));
+            const double pv[3] = {A.rec[i].px, A.rec[i].py, A.rec[i].pz};
+            double ri[3], zi[3], di[3], m[6], yi[3] = {0, 0, 0};
+            bool sk[3];
+            for (int c = 0; c < 3; c++) {
+                ri[c] = A.r[i + c * n];
+                di[c] = A.d[i + c * n];
+                sk[c] = A.skip[i + c * n] != 0;
+            }
+            for (int c = 0; c < 6; c++) m[c] = A.Minv[i + c * n];
+            for (int q = q2.x; q < q2.y; q += 4) {
+                const double *ys = A.yseg + (int64_t)q * 96 + (i & 31);
+                double v[4][3];
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) v[k][c] = q + k < q2.y ? __ldcg(ys + k * 96 + c * 32) : 0.0;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) yi[c] += v[k][c];
+            }
+            for (int c = 0; c < 3; c++) {
+                A.d[i + c * n] = di[c] + alpha * pv[c];
+                ri[c] = sk[c] ? 0.0 : ri[c] - alpha * yi[c];
+                A.r[i + c * n] = ri[c];
+            }
+            apply_minv(m, ri, zi);
+            for (int c = 0; c < 3; c++) {
+                if (sk[c]) zi[c] = 0.0;
+                A.z[i + c * n] = zi[c];
+                rzn += ri[c] * zi[c];
+                rrn += ri[c] * ri[c];
+            }
+        }
+        if (!grid_sum2(rzn, rrn, sh, part0, bar)) return;
+        // p = z + beta p
+        const double beta = rz != 0 ? rzn / rz : 0.0;
+        GRID_STRIDE(i, n)
+        {
+            A.rec[i].px = A.z[i] + beta * A.rec[i].px;
+            A.rec[i].py = A.z[i + n] + beta * A.rec[i].py;
+            A.rec[i].pz = A.z[i + 2 * n] + beta * A.rec[i].pz;
+        }
+        rz = rzn;
+        rr = rrn;
+        done++;
+        if (done % kCgCheck == 0 || done == A.max_cg) {
+            if (!isfinite(rr)) state = CG_NONFINITE;
+            else if (rr <= A.tol2 * rr0 || done == A.max_cg) state = CG_DONE;
+        }
+        if (state == CG_MORE && !bar.wait()) return;
+    }
+    if (state == CG_DONE)
+        GRID_STRIDE(i, n)
+            for (int c = 0; c < 3; c++) A.x[i + c * n] += A.d[i + c * n];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.scal[0] = rz;
+        A.scal[1] = rr;
+        A.scal[2] = rr0;
+        A.state[0] = state;
+        A.state[1] = done;
     }
 }
-
-// p = z + beta p with beta = (new r.z) / (old r.z); rolls r.z forward
-__global__ void k_cg_direction(int64_t n, const double *__restrict__ z, double *p, const double *__restrict__ rzn,
-                               const double *__restrict__ scal)
-{
-    const double beta = scal[0] != 0 ? rzn[0] / scal[0] : 0.0;
-    GRID_STRIDE(e, 3 * n) p[e] = z[e] + beta * p[e];
-}
-
-__global__ void k_roll(double *scal, const double *__restrict__ rzn)
-{
-    if (threadIdx.x == 0) {
-        scal[0] = rzn[0];
-        scal[1] = rzn[1];
-    }
-}
-
-__global__ void k_move(int64_t m, double *x, const double *__restrict__ d) { GRID_STRIDE(e, m) x[e] += d[e]; }
 
 __global__ void k_prescribe(int64_t m, double *x, const uint8_t *__restrict__ held, double inc)
 {
@@ -435,12 +636,18 @@ struct bbpd_static {
     int64_t n = 0, nB = 0;
     bbpd_params prm{};
     std::vector<void *> allocs;
-    double *X = nullptr, *x = nullptr, *F = nullptr, *d = nullptr, *r = nullptr, *z = nullptr, *p = nullptr,
-           *Kp = nullptr, *Minv = nullptr, *part = nullptr, *scal = nullptr, *rzn = nullptr, *red = nullptr;
+    double *X = nullptr, *x = nullptr, *F = nullptr, *d = nullptr, *r = nullptr, *z = nullptr,
+           *Minv = nullptr, *part = nullptr, *scal = nullptr, *red = nullptr, *rigE = nullptr;
+    NodeRec *rec = nullptr;
+    double2 *cg_part = nullptr;
+    int *cg_state = nullptr;               // state, iterations, error word, barrier arrivals
+    int cg_grid = 0;
+    int64_t rows = 0, chunk = 1;
+    double *yseg = nullptr;
+    int32_t *seg = nullptr;
     uint8_t *skip = nullptr;
     SBonds b{};
     SNodes g{};
-    cudaGraphExec_t cg_exec = nullptr;   // kCgBlock conjugate-gradient iterations, captured once
     template <class T>
     int alloc(T **q, size_t count)
     {
@@ -451,7 +658,6 @@ struct bbpd_static {
     ~bbpd_static()
     {
         if (st) cudaStreamSynchronize(st);
-        if (cg_exec) cudaGraphExecDestroy(cg_exec);
         for (void *q : allocs) cudaFree(q);
         if (st) cudaStreamDestroy(st);
     }
@@ -459,43 +665,27 @@ struct bbpd_static {
 
 namespace {
 
-constexpr int kCgBlock = 8;   // iterations between convergence checks
-
-// `iters` conjugate-gradient iterations; the step sizes live in device memory,
-// so nothing here waits for the host
-void enqueue_cg(bbpd_static *S, int iters)
+// K delta = F on the free DOFs and x += delta; iterations and the outcome in
+// state[0..1]. The host looks at the outcome once per launch.
+int run_cg(bbpd_static *S, double cg_tol, int max_cg, int state[2])
 {
     cudaStream_t st = S->st;
-    const int64_t n = S->n;
-    for (int c = 0; c < iters; c++) {
-        k_static_spmv<<<kRedBlocks, kThreads, 0, st>>>(S->g, S->b.a, S->b.b, S->b.rig, S->b.c, S->p, S->Kp, S->part);
-        k_reduce<<<1, 32, 0, st>>>(S->part, kRedBlocks, 1, S->scal + 2);
-        k_cg_update<<<kRedBlocks, kThreads, 0, st>>>(n, S->skip, S->Minv, S->scal, S->p, S->Kp, S->d, S->r, S->z,
-                                                     S->part);
-        k_reduce<<<1, 32, 0, st>>>(S->part, kRedBlocks, 2, S->rzn);
-        k_cg_direction<<<blocks_for(3 * n), kThreads, 0, st>>>(n, S->z, S->p, S->rzn, S->scal);
-        k_roll<<<1, 32, 0, st>>>(S->scal, S->rzn);
+    const double to = S->prm.barrier_timeout_s > 0 ? S->prm.barrier_timeout_s : 2.0;
+    CgArgs A{S->g, S->rigE, S->rec, S->F, S->Minv, S->skip, S->x, S->d, S->r, S->z, S->yseg, S->seg, S->cg_part,
+             S->scal, S->cg_state, reinterpret_cast<unsigned *>(S->cg_state + 3), (unsigned long long)(to * 1e9),
+             cg_tol * cg_tol, 1, max_cg, S->rows, S->chunk};
+    for (;; A.first = 0) {
+        BBPD_CUDA_TRY(cudaMemsetAsync(S->cg_state + 2, 0, 2 * sizeof(int), st));
+        void *args[] = {(void *)&A};
+        BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_cg, dim3(S->cg_grid), dim3(kCgThreads), args, 0, st));
+        int h[3];
+        BBPD_CUDA_TRY(cudaMemcpyAsync(h, S->cg_state, sizeof(h), cudaMemcpyDeviceToHost, st));
+        BBPD_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h[2] & ERR_TIMEOUT) return fail(BBPD_ERR_TIMEOUT, "grid barrier wait exceeded its limit; kernel returned early");
+        state[0] = h[0];
+        state[1] = h[1];
+        if (h[0] != CG_MORE) return BBPD_OK;
     }
-}
-
-// kCgBlock iterations as one graph launch (the 6 kernels of an iteration are
-// launch-bound on small problems); captured on first use
-int run_cg_block(bbpd_static *S)
-{
-    if (!S->cg_exec) {
-        cudaGraph_t gr = nullptr;
-        BBPD_CUDA_TRY(cudaStreamBeginCapture(S->st, cudaStreamCaptureModeThreadLocal));
-        enqueue_cg(S, kCgBlock);
-        cudaError_t e = cudaStreamEndCapture(S->st, &gr);
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&S->cg_exec, gr, 0);
-        if (gr) cudaGraphDestroy(gr);
-        if (e != cudaSuccess) {
-            S->cg_exec = nullptr;
-            return fail(BBPD_ERR_CUDA, "conjugate-gradient graph: %s", cudaGetErrorString(e));
-        }
-    }
-    BBPD_CUDA_TRY(cudaGraphLaunch(S->cg_exec, S->st));
-    return BBPD_OK;
 }
 
 int read_scalars(bbpd_static *S, const double *src, int cnt, double *out)
@@ -569,12 +759,12 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     TRY(S->alloc(&S->x, 3 * n));
     TRY(staging::upload_copy(S->X, pb->undeformed_coordinates, 3 * n, st));
     BBPD_CUDA_TRY(cudaMemcpyAsync(S->x, S->X, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, st));
-    for (double **q : {&S->F, &S->d, &S->r, &S->z, &S->p, &S->Kp}) TRY(S->alloc(q, 3 * n));
+    for (double **q : {&S->F, &S->d, &S->r, &S->z}) TRY(S->alloc(q, 3 * n));
+    TRY(S->alloc(&S->rec, n));
     TRY(S->alloc(&S->Minv, 6 * n));
     TRY(S->alloc(&S->skip, 3 * n));
     TRY(S->alloc(&S->part, 2 * kRedBlocks));
     TRY(S->alloc(&S->scal, 4));
-    TRY(S->alloc(&S->rzn, 2));
     TRY(S->alloc(&S->red, 2));
     BBPD_CUDA_TRY(cudaMemsetAsync(S->F, 0, sizeof(double) * 3 * n, st));
 
@@ -593,7 +783,6 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     TRY(S->alloc(&B.bsf, nB));
     TRY(S->alloc(&B.flag, nB));
     TRY(S->alloc(&B.rig, nB));
-    TRY(S->alloc(&B.c, 3 * nB));
     TRY(S->alloc(&B.f, 3 * nB));
     TRY(S->alloc(&dheld, 3 * n));
     TRY(staging::upload_copy(da, a.data(), nB, st));
@@ -634,7 +823,7 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     P.ff = prm->failure_functionality;
 
     // per-node lists of bond ends in bond order: stable sort of q = 2k + side by node
-    const int64_t m = 2 * nB;
+    const int64_t m = 2 * nB;   // list entries
     int64_t *off = nullptr;
     uint32_t *ent = nullptr;
     TRY(S->alloc(&off, n + 1));
@@ -680,8 +869,58 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
             cudaFreeAsync(q, st);
         TRY(rc);
     }
+    // the same lists in slices of 32 nodes
+    const int64_t ns = (n + 31) / 32;
+    int64_t *sptr = nullptr, slots = 0;
+    uint32_t *bond = nullptr, *col = nullptr;
+    TRY(S->alloc(&sptr, ns + 1));
+    {
+        int64_t *cnt = nullptr;
+        uint8_t *tmp = nullptr;
+        size_t tb = 0;
+        BBPD_CUDA_TRY(cudaMallocAsync(&cnt, sizeof(int64_t) * (ns + 1), st));
+        k_slice_lengths<<<blocks_for(32 * (ns + 1)), kThreads, 0, st>>>(off, n, ns, cnt);
+        cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, sptr, ns + 1, st);
+        if (e == cudaSuccess) e = cudaMallocAsync(&tmp, std::max<size_t>(tb, 1), st);
+        if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, sptr, ns + 1, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&slots, sptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        cudaFreeAsync(cnt, st);
+        if (tmp) cudaFreeAsync(tmp, st);
+        if (e != cudaSuccess) return fail(BBPD_ERR_CUDA, "static solver slices: %s", cudaGetErrorString(e));
+    }
+    TRY(S->alloc(&bond, slots));
+    TRY(S->alloc(&col, slots));
+    TRY(S->alloc(&S->rigE, slots));
+    k_slice_fill<<<blocks_for(32 * ns), kThreads, 0, st>>>(off, ent, da, db, n, ns, sptr, bond, col);
+    TRY(launch_check());
+    int nsm = 0, occ = 0, coop = 0;
+    BBPD_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+    BBPD_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    if (!coop) return fail(BBPD_ERR_UNSUPPORTED, "device lacks cooperative launch");
+    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg, kCgThreads, 0));
+    if (occ < 1) return fail(BBPD_ERR_CUDA, "kernel cannot be resident");
+    // no more blocks than give every warp four rows, and every thread a node
+    const int64_t wpb = kCgThreads / 32;
+    S->rows = slots / 32;
+    S->cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * occ,
+                                                             std::max((S->rows + 4 * wpb - 1) / (4 * wpb),
+                                                                      (n + kCgThreads - 1) / kCgThreads)));
+    S->chunk = std::max<int64_t>(1, (S->rows + S->cg_grid * wpb - 1) / (S->cg_grid * wpb));
+    TRY(S->alloc(&S->yseg, (ns + S->cg_grid * wpb) * 96));
+    TRY(S->alloc(&S->seg, 2 * ns));
+    k_segments<<<blocks_for(ns), kThreads, 0, st>>>(sptr, ns, S->chunk, S->seg);
+    TRY(launch_check());
+    TRY(S->alloc(&S->cg_part, 2 * S->cg_grid));
+    TRY(S->alloc(&S->cg_state, 4));
     S->g.off = off;
     S->g.ent = ent;
+    S->g.a = da;
+    S->g.b = db;
+    S->g.sptr = sptr;
+    S->g.bond = bond;
+    S->g.col = col;
+    S->g.ns = ns;
     S->g.held = dheld;
     S->g.n = n;
     S->g.nB = nB;
@@ -704,7 +943,7 @@ extern "C" int bbpd_static_step(bbpd_static *S, double increment, double tol, in
     for (int it = 0;; it++) {
         k_static_bonds<<<blocks_for(S->nB), kThreads, 0, st>>>(S->b, S->x, n);
         k_static_nodal<<<kRedBlocks, kThreads, 0, st>>>(S->g, S->b.f, S->prm.cell_volume, S->F, S->part);
-        k_reduce<<<1, 32, 0, st>>>(S->part, kRedBlocks, 2, S->red);
+        k_reduce<<<1, 64, 0, st>>>(S->part, kRedBlocks, 2, S->red);
         TRY(launch_check());
         double rr[2];
         TRY(read_scalars(S, S->red, 2, rr));
@@ -718,30 +957,15 @@ extern "C" int bbpd_static_step(bbpd_static *S, double increment, double tol, in
             return BBPD_OK;
         }
         if (it == max_newton) return BBPD_OK;   // not converged: stats say so
-        // K delta = F on the free DOFs by PCG
-        k_static_precond<<<blocks_for(n), kThreads, 0, st>>>(S->g, S->b.a, S->b.b, S->b.rig, S->b.c, S->Minv, S->skip);
-        k_cg_init<<<kRedBlocks, kThreads, 0, st>>>(n, S->F, S->skip, S->Minv, S->d, S->r, S->z, S->p, S->part);
-        k_reduce<<<1, 32, 0, st>>>(S->part, kRedBlocks, 2, S->scal);
+        // K delta = F on the free DOFs by PCG, x += delta
+        k_static_records<<<blocks_for(n), kThreads, 0, st>>>(S->x, n, S->rec);
+        k_slot_rig<<<blocks_for(2 * S->nB), kThreads, 0, st>>>(S->g.bond, S->b.rig, S->g.sptr + S->g.ns, S->rigE);
+        k_static_precond<<<blocks_for(32 * n), kThreads, 0, st>>>(S->g, S->b.rig, S->rec, S->Minv, S->skip);
         TRY(launch_check());
-        double s01[2];
-        TRY(read_scalars(S, S->scal, 2, s01));
-        const double rr0 = s01[1];
-        if (rr0 > 0) {
-            for (int done = 0; done < max_cg;) {
-                const int blk = std::min(kCgBlock, max_cg - done);
-                if (blk == kCgBlock) TRY(run_cg_block(S));
-                else enqueue_cg(S, blk);
-                TRY(launch_check());
-                done += blk;
-                stats->cg_iterations += blk;
-                double rz[2];
-                TRY(read_scalars(S, S->rzn, 2, rz));
-                if (!std::isfinite(rz[1])) return fail(BBPD_ERR_NONFINITE, "conjugate gradient diverged");
-                if (rz[1] <= cg_tol * cg_tol * rr0) break;
-            }
-        }
-        k_move<<<blocks_for(3 * n), kThreads, 0, st>>>(3 * n, S->x, S->d);
-        TRY(launch_check());
+        int cg[2] = {CG_DONE, 0};
+        TRY(run_cg(S, cg_tol, max_cg, cg));
+        stats->cg_iterations += cg[1];
+        if (cg[0] == CG_NONFINITE) return fail(BBPD_ERR_NONFINITE, "conjugate gradient diverged");
     }
 }
 

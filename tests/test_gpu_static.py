@@ -130,3 +130,30 @@ def test_static_other_laws_vs_oracle(law, steps):
         assert same_flags(g.get("fail"), o.get("fail")), step
     assert g.get("flag").sum() > 100
     g.close()
+
+
+# half a slice, a ragged last slice, more rows than warps, and a beam whose last
+# 70 nodes have lost their bonds (slices without a row)
+@pytest.mark.parametrize("nx,ny,nz,cut", [(6, 2, 2, 0), (13, 3, 5, 0), (40, 6, 8, 0), (30, 4, 6, 70)])
+def test_static_solve_sizes_vs_oracle(nx, ny, nz, cut):
+    """The linear solve where its rows, slices and segments meet differently."""
+    inp = dict(bb.beam.build(bb.beam.small(nx=nx, ny=ny, nz=nz)))
+    if cut:   # the top layer's end, away from the loaded nodes
+        keep = (inp["BONDLIST"] <= inp["nNodes"] - cut).all(axis=1)
+        moved = np.nonzero(inp["BODYFORCEFLAG"].any(axis=1))[0]
+        inp["BODYFORCEFLAG"] = inp["BODYFORCEFLAG"].copy(order="F")
+        inp["BODYFORCEFLAG"][moved] = 0
+        inp["BODYFORCEFLAG"][moved - cut, 2] = 1   # load nodes that keep their bonds
+        for k in ("UNDEFORMEDLENGTH", "BONDSTIFFNESS", "VOLUMECORRECTIONFACTORS"):
+            inp[k] = inp[k][keep].copy()
+        inp["BONDLIST"] = np.asfortranarray(inp["BONDLIST"][keep])
+        inp["nBonds"] = int(keep.sum())
+    g = StaticSolver(inp, law="linear", sc=1.0)
+    o = StaticOracle(inp, law="linear", sc=1.0)
+    for step in range(2):
+        sg = g.step(-1e-6, tol=1e-9, **CG)
+        so = o.step(-1e-6, tol=1e-9)
+        assert sg.converged and so["converged"], (step, sg.residual, sg.reaction)
+        ug, uo = g.get("displacement"), o.get("displacement")
+        assert np.abs(ug - uo).max() <= 1e-8 * np.abs(uo).max(), step
+    g.close()
