@@ -10,14 +10,20 @@
 // Horizons. The nodes are binned into a uniform grid whose cell edge is the
 // horizon widened by 1e-6 (so rounding in the binning never puts two nodes
 // within the horizon more than one cell apart) and sorted by cell with a radix
-// sort. Every node scans the 27 cells around its own and keeps each j != i with
-// sqrt(((xi-xj)^2 + (yi-yj)^2) + (zi-zj)^2) <= horizon: the expression of the
-// reference's UNDEFORMEDLENGTH, so the test and the stored length agree bit for
-// bit (the squared differences are the same both ways, so the relation is
-// symmetric). A count pass sizes the families, a fill pass writes (i, j) keys,
-// and a radix sort of the keys lists every family by ascending node id (the
-// reference's rangesearch lists them by distance; both are valid families).
-// Bonds are the pairs with j > i, by i then j.
+// sort, their positions with them. Every node scans the 27 cells around its own
+// (nine runs of three cells that lie in a row in the sorted order) and keeps each
+// j != i with sqrt(((xi-xj)^2 + (yi-yj)^2) + (zi-zj)^2) <= horizon: the expression
+// of the reference's UNDEFORMEDLENGTH, so the test and the stored length agree bit
+// for bit (the squared differences are the same both ways, so the relation is
+// symmetric). A count pass sizes the families; a fill pass finds them again and
+// lists each by ascending node id (the reference's rangesearch lists them by
+// distance; both are valid families). Bonds are the pairs with j > i, by i then j.
+//
+// A warp takes a node, its lanes 32 candidates: a thread per node left most SMs of a
+// small cloud idle and walked some 700 candidates one after the other. The fill
+// pass ranks the members of a family within the warp and writes them in place;
+// families of more than kRankMax members go through (i, j) keys and a global radix
+// sort instead.
 //
 // Notch. The rectangle's corners and unit normal are formed on the host
 // exactly as determineintersection.m forms them; one thread per bond runs the
@@ -28,7 +34,6 @@
 #include "staging.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
 
@@ -111,58 +116,102 @@ __global__ void k_cell_of(const double *__restrict__ X, int64_t n, Grid g, uint3
     }
 }
 
-__global__ void k_cell_bounds(const uint32_t *__restrict__ scell, int64_t n, uint32_t *first, uint32_t *last)
+// start[c]: first sorted position whose cell is c or later, for c in [0, ncell]
+__global__ void k_cell_starts(const uint32_t *__restrict__ scell, int64_t n, int64_t ncell, uint32_t *start)
 {
-    GRID_STRIDE(q, n)
+    GRID_STRIDE(q, n + 1)
     {
-        const uint32_t c = scell[q];
-        if (q == 0 || scell[q - 1] != c) first[c] = (uint32_t)q;
-        if (q == n - 1 || scell[q + 1] != c) last[c] = (uint32_t)(q + 1);
+        const int64_t c0 = q == 0 ? 0 : (int64_t)scell[q - 1] + 1, c1 = q == n ? ncell : (int64_t)scell[q];
+        for (int64_t c = c0; c <= c1; c++) start[c] = (uint32_t)q;
     }
 }
 
-// FILL = false: family size and forward (j > i) count of every node.
-// FILL = true: the (i, j) keys of every family, unordered within it.
-template <bool FILL>
-__global__ void k_horizon_scan(const double *__restrict__ X, int64_t n, double horizon, Grid g,
-                               const uint32_t *__restrict__ scell, const uint32_t *__restrict__ snode,
-                               const uint32_t *__restrict__ first, const uint32_t *__restrict__ last,
-                               int32_t *fam, int32_t *fwd, const int64_t *__restrict__ famoff, int bits,
-                               uint64_t *keys)
+// positions in sorted order
+__global__ void k_sorted_positions(const double *__restrict__ X, int64_t n, const uint32_t *__restrict__ snode, double *sx)
 {
     GRID_STRIDE(q, n)
     {
         const int64_t i = snode[q];
-        const int64_t c = scell[q];
-        const int64_t cx = c % g.nc[0], cy = (c / g.nc[0]) % g.nc[1], cz = c / (g.nc[0] * g.nc[1]);
-        int32_t nf = 0, nfw = 0;
-        int64_t out = FILL ? famoff[i] : 0;
-        const int64_t end = FILL ? famoff[i + 1] : 0;   // the count pass sized this family
-        for (int64_t z = cz - 1; z <= cz + 1; z++) {
-            if (z < 0 || z >= g.nc[2]) continue;
-            for (int64_t y = cy - 1; y <= cy + 1; y++) {
-                if (y < 0 || y >= g.nc[1]) continue;
-                for (int64_t x = cx - 1; x <= cx + 1; x++) {
-                    if (x < 0 || x >= g.nc[0]) continue;
-                    const int64_t cc = x + g.nc[0] * (y + g.nc[1] * z);
-                    const uint32_t a = first[cc], b = last[cc];
-                    for (uint32_t r = a; r < b; r++) {
-                        const int64_t j = snode[r];
-                        if (j == i || !(pair_length(X, n, i, j) <= horizon)) continue;
-                        if (FILL) {
-                            if (out < end) keys[out++] = ((uint64_t)i << bits) | (uint64_t)j;
-                        } else {
-                            nf++;
-                            nfw += j > i;
-                        }
-                    }
+        sx[q] = X[i];
+        sx[q + n] = X[i + n];
+        sx[q + 2 * n] = X[i + 2 * n];
+    }
+}
+
+struct Cloud {
+    int64_t n;
+    double horizon;
+    Grid g;
+    const uint32_t *scell, *snode, *start;
+    const double *sx;   // positions in sorted order, x then y then z
+};
+
+// Every candidate of the node at sorted position q, 32 at a time: found(hit, j,
+// L) with lane's candidate j and its distance, hit where it is in the family.
+template <class F>
+__device__ __forceinline__ void scan_family(const Cloud &C, int64_t q, int lane, F found)
+{
+    const int64_t n = C.n, i = C.snode[q], c = C.scell[q];
+    const double xi = C.sx[q], yi = C.sx[q + n], zi = C.sx[q + 2 * n];
+    const int64_t nx = C.g.nc[0], ny = C.g.nc[1], nz = C.g.nc[2];
+    const int64_t cx = c % nx, cy = (c / nx) % ny, cz = c / (nx * ny);
+    const int64_t xa = cx > 0 ? cx - 1 : 0, xb = cx + 1 < nx ? cx + 1 : nx - 1;
+    for (int64_t z = cz > 0 ? cz - 1 : 0; z <= cz + 1 && z < nz; z++)
+        for (int64_t y = cy > 0 ? cy - 1 : 0; y <= cy + 1 && y < ny; y++) {
+            const int64_t row = nx * (y + ny * z);
+            const uint32_t a = C.start[row + xa], b = C.start[row + xb + 1];
+            for (uint32_t r0 = a; r0 < b; r0 += 32) {
+                const uint32_t r = r0 + lane;
+                int64_t j = i;
+                double L = 0;
+                if (r < b) {
+                    j = C.snode[r];
+                    const double e0 = xi - C.sx[r], e1 = yi - C.sx[r + n], e2 = zi - C.sx[r + 2 * n];
+                    L = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
                 }
+                found(r < b && j != i && L <= C.horizon, j, L);
             }
         }
-        if (!FILL) {
+}
+
+// Family size and forward (j > i) count of every node, and the largest family.
+__global__ void __launch_bounds__(kThreads) k_horizon_count(Cloud C, int32_t *fam, int32_t *fwd, int *largest)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    int most = 0;
+    for (int64_t q = (blockIdx.x * (int64_t)kThreads + threadIdx.x) >> 5; q < C.n; q += warps) {
+        const int64_t i = C.snode[q];
+        int nf = 0, nfw = 0;
+        scan_family(C, q, lane, [&](bool hit, int64_t j, double) {
+            nf += __popc(__ballot_sync(0xffffffffu, hit));
+            nfw += __popc(__ballot_sync(0xffffffffu, hit && j > i));
+        });
+        if (lane == 0) {
             fam[i] = nf;
             fwd[i] = nfw;
         }
+        most = max(most, nf);
+    }
+    if (lane == 0) atomicMax(largest, most);
+}
+
+// The (i, j) keys of every family, unordered within it (families too large to
+// rank in a warp).
+__global__ void __launch_bounds__(kThreads) k_horizon_keys(Cloud C, const int64_t *__restrict__ famoff, int bits,
+                                                           uint64_t *keys)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    for (int64_t q = (blockIdx.x * (int64_t)kThreads + threadIdx.x) >> 5; q < C.n; q += warps) {
+        const int64_t i = C.snode[q], end = famoff[i + 1];   // the count pass sized this family
+        int64_t out = famoff[i];
+        scan_family(C, q, lane, [&](bool hit, int64_t j, double) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            const int64_t at = out + __popc(m & ((1u << lane) - 1));
+            if (hit && at < end) keys[at] = ((uint64_t)i << bits) | (uint64_t)j;
+            out += __popc(m);
+        });
     }
 }
 
@@ -196,6 +245,60 @@ __global__ void k_horizon_emit(const uint64_t *__restrict__ skeys, int64_t nf, i
             o.bl[b + o.nb] = (double)(j + 1);
             o.L0[b] = pair_length(X, n, i, j);
         }
+    }
+}
+
+// Every family found again and written by ascending node id: the warp keeps its
+// members in shared memory and each member's rank is the number of smaller ids.
+constexpr int kRankMax = 256;
+
+__global__ void __launch_bounds__(kThreads) k_horizon_fill(Cloud C, const int64_t *__restrict__ famoff,
+                                                           const int64_t *__restrict__ boff, HorizonOut o)
+{
+    __shared__ double s_len[kThreads / 32][kRankMax];
+    __shared__ __align__(16) uint32_t s_id[kThreads / 32][kRankMax];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    for (int64_t q = (blockIdx.x * (int64_t)kThreads + threadIdx.x) >> 5; q < C.n; q += warps) {
+        const int64_t i = C.snode[q], f0 = famoff[i], b0 = boff[i];
+        const int nf = (int)(famoff[i + 1] - f0), back = nf - (int)(boff[i + 1] - b0);   // members below i
+        int got = 0;
+        scan_family(C, q, lane, [&](bool hit, int64_t j, double L) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit);
+            const int at = got + __popc(m & ((1u << lane) - 1));
+            if (hit && at < nf) {   // the count pass sized this family, at most kRankMax
+                s_id[w][at] = (uint32_t)j;
+                s_len[w][at] = L;
+            }
+            got += __popc(m);
+        });
+        if (lane < 4 && nf + lane < kRankMax) s_id[w][nf + lane] = 0xFFFFFFFFu;   // pads the last group of four
+        __syncwarp();
+        for (int m0 = 0; m0 < nf; m0 += 128) {
+            uint32_t id[4];
+            int rank[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int k = 0; k < 4; k++) id[k] = m0 + 32 * k + lane < nf ? s_id[w][m0 + 32 * k + lane] : 0u;
+            for (int t = 0; t < nf; t += 4) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(&s_id[w][t]);
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    rank[k] += (v.x < id[k]) + (v.y < id[k]) + (v.z < id[k]) + (v.w < id[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int at = m0 + 32 * k + lane;
+                if (at >= nf) continue;
+                if (o.family) o.family[f0 + rank[k]] = (double)id[k] + 1.0;
+                if (o.bl && rank[k] >= back) {
+                    const int64_t b = b0 + (rank[k] - back);
+                    o.bl[b] = (double)(i + 1);
+                    o.bl[b + o.nb] = (double)id[k] + 1.0;
+                    o.L0[b] = s_len[w][at];
+                }
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -343,10 +446,53 @@ __global__ void k_massmatrix(const double *__restrict__ nfam, int64_t n, double 
     }
 }
 
-__global__ void k_nonfinite(const double *__restrict__ X, int64_t n, int *bad)
+// Least and greatest value of every coordinate column, and whether one is not
+// finite: block partials, folded by the block that finishes last. out: lo[3],
+// hi[3], then the flag. *arrived must be 0.
+constexpr int kBoundsBlocks = 148;
+
+__global__ void __launch_bounds__(kThreads) k_bounds(const double *__restrict__ X, int64_t n, double *part,
+                                                     unsigned *arrived, double *out)
 {
+    __shared__ double sh[7][kThreads / 32];
+    __shared__ bool s_last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double v[7] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0.0};
+    auto fold = [&]() {   // the block's values, in thread 0
+        for (int o = 16; o > 0; o >>= 1)
+            for (int k = 0; k < 7; k++) {
+                const double u = __shfl_xor_sync(0xffffffffu, v[k], o);
+                v[k] = k < 3 ? fmin(v[k], u) : fmax(v[k], u);
+            }
+        if (lane == 0)
+            for (int k = 0; k < 7; k++) sh[k][w] = v[k];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int q = 1; q < kThreads / 32; q++)
+                for (int k = 0; k < 7; k++) v[k] = k < 3 ? fmin(v[k], sh[k][q]) : fmax(v[k], sh[k][q]);
+    };
     GRID_STRIDE(i, n)
-    if (!isfinite(X[i])) *bad = 1;
+        for (int a = 0; a < 3; a++) {
+            const double x = X[i + a * n];
+            if (!isfinite(x)) v[6] = 1.0;
+            v[a] = fmin(v[a], x);
+            v[3 + a] = fmax(v[3 + a], x);
+        }
+    fold();
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 7; k++) part[7 * blockIdx.x + k] = v[k];
+        __threadfence();
+        s_last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const bool in = threadIdx.x < gridDim.x;
+    for (int k = 0; k < 7; k++)
+        v[k] = in ? __ldcg(&part[7 * threadIdx.x + k]) : (k < 3 ? INFINITY : k < 6 ? -INFINITY : 0.0);
+    fold();
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 7; k++) out[k] = v[k];
 }
 
 // min and max of every coordinate column: six values to the host; fails on a
@@ -354,34 +500,17 @@ __global__ void k_nonfinite(const double *__restrict__ X, int64_t n, int *bad)
 int coord_bounds(const double *X, int64_t n, cudaStream_t st, double lo[3], double hi[3])
 {
     Scratch s(st);
-    double *out = nullptr;
-    int *bad = nullptr;
-    TRY(s.get(&out, 6));
-    TRY(s.get(&bad, 1));
-    BBPD_CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), st));
-    k_nonfinite<<<blocks_for(3 * n), kThreads, 0, st>>>(X, 3 * n, bad);
+    double *part = nullptr;   // block partials, result, arrivals
+    TRY(s.get(&part, 7 * kBoundsBlocks + 8));
+    double *out = part + 7 * kBoundsBlocks;
+    unsigned *arrived = reinterpret_cast<unsigned *>(out + 7);
+    BBPD_CUDA_TRY(cudaMemsetAsync(arrived, 0, sizeof(unsigned), st));
+    k_bounds<<<std::min(kBoundsBlocks, blocks_for(n)), kThreads, 0, st>>>(X, n, part, arrived, out);
     TRY(launch_check());
-    size_t tb = 0, tmax = 0;
-    for (int a = 0; a < 3; a++) {
-        BBPD_CUDA_TRY(cub::DeviceReduce::Min(nullptr, tb, X + a * n, out + a, n, st));
-        tmax = std::max(tmax, tb);
-        BBPD_CUDA_TRY(cub::DeviceReduce::Max(nullptr, tb, X + a * n, out + 3 + a, n, st));
-        tmax = std::max(tmax, tb);
-    }
-    uint8_t *tmp = nullptr;
-    TRY(s.get(&tmp, tmax));
-    for (int a = 0; a < 3; a++) {
-        tb = tmax;
-        BBPD_CUDA_TRY(cub::DeviceReduce::Min(tmp, tb, X + a * n, out + a, n, st));
-        tb = tmax;
-        BBPD_CUDA_TRY(cub::DeviceReduce::Max(tmp, tb, X + a * n, out + 3 + a, n, st));
-    }
-    double h[6];
-    int hb = 0;
+    double h[7];
     BBPD_CUDA_TRY(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, st));
-    BBPD_CUDA_TRY(cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
     BBPD_CUDA_TRY(cudaStreamSynchronize(st));
-    if (hb) return fail(BBPD_ERR_ARG, "coordinates must be finite");
+    if (h[6] != 0) return fail(BBPD_ERR_ARG, "coordinates must be finite");
     for (int a = 0; a < 3; a++) {
         lo[a] = h[a];
         hi[a] = h[3 + a];
@@ -403,7 +532,8 @@ struct Horizons {
     double horizon = 0;
     int bits = 1;
     Grid g{};
-    uint32_t *scell = nullptr, *snode = nullptr, *first = nullptr, *last = nullptr;
+    Cloud C{};
+    int largest = 0;   // members of the largest family
     int32_t *fam = nullptr, *fwd = nullptr;
     int64_t *famoff = nullptr, *boff = nullptr;
     explicit Horizons(cudaStream_t s_) : st(s_), s(s_) {}
@@ -431,7 +561,9 @@ struct Horizons {
             g.h *= 1.25;
         }
         const int64_t ncell = g.nc[0] * g.nc[1] * g.nc[2];
-        uint32_t *cell = nullptr, *node = nullptr;
+        uint32_t *cell = nullptr, *node = nullptr, *scell = nullptr, *snode = nullptr, *start = nullptr;
+        double *sx = nullptr;
+        int *dlargest = nullptr;
         TRY(s.get(&cell, n));
         TRY(s.get(&node, n));
         TRY(s.get(&scell, n));
@@ -443,16 +575,17 @@ struct Horizons {
         uint8_t *tmp = nullptr;
         TRY(s.get(&tmp, tb));
         BBPD_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, cell, scell, node, snode, n, 0, bits_for(ncell), st));
-        TRY(s.get(&first, ncell));
-        TRY(s.get(&last, ncell));
-        BBPD_CUDA_TRY(cudaMemsetAsync(first, 0, sizeof(uint32_t) * ncell, st));
-        BBPD_CUDA_TRY(cudaMemsetAsync(last, 0, sizeof(uint32_t) * ncell, st));
-        k_cell_bounds<<<blocks_for(n), kThreads, 0, st>>>(scell, n, first, last);
+        TRY(s.get(&start, ncell + 1));
+        TRY(s.get(&sx, 3 * n));
+        k_cell_starts<<<blocks_for(n + 1), kThreads, 0, st>>>(scell, n, ncell, start);
+        k_sorted_positions<<<blocks_for(n), kThreads, 0, st>>>(X, n, snode, sx);
         TRY(launch_check());
         TRY(s.get(&fam, n));
         TRY(s.get(&fwd, n));
-        k_horizon_scan<false><<<blocks_for(n), kThreads, 0, st>>>(X, n, r, g, scell, snode, first, last, fam, fwd,
-                                                                  nullptr, bits, nullptr);
+        TRY(s.get(&dlargest, 1));
+        BBPD_CUDA_TRY(cudaMemsetAsync(dlargest, 0, sizeof(int), st));
+        C = Cloud{n, r, g, scell, snode, start, sx};
+        k_horizon_count<<<blocks_for(32 * n), kThreads, 0, st>>>(C, fam, fwd, dlargest);
         TRY(launch_check());
         int64_t *w = nullptr;
         TRY(s.get(&w, n + 1));
@@ -468,6 +601,7 @@ struct Horizons {
         TRY(launch_check());
         BBPD_CUDA_TRY(cudaMemcpyAsync(&nf, famoff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         BBPD_CUDA_TRY(cudaMemcpyAsync(&nb, boff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        BBPD_CUDA_TRY(cudaMemcpyAsync(&largest, dlargest, sizeof(int), cudaMemcpyDeviceToHost, st));
         BBPD_CUDA_TRY(cudaStreamSynchronize(st));
         if (nf != 2 * nb) return fail(BBPD_ERR_CUDA, "horizon search: %lld family entries for %lld bonds",
                                       (long long)nf, (long long)nb);
@@ -484,18 +618,21 @@ struct Horizons {
     int emit(HorizonOut o)
     {
         if (nf == 0 || (!o.family && !o.bl)) return BBPD_OK;
+        o.nb = nb;
+        if (largest <= kRankMax) {
+            k_horizon_fill<<<blocks_for(32 * n), kThreads, 0, st>>>(C, famoff, boff, o);
+            return launch_check();
+        }
         uint64_t *keys = nullptr, *skeys = nullptr;
         TRY(s.get(&keys, nf));
         TRY(s.get(&skeys, nf));
-        k_horizon_scan<true><<<blocks_for(n), kThreads, 0, st>>>(X, n, horizon, g, scell, snode, first, last, fam,
-                                                                 fwd, famoff, bits, keys);
+        k_horizon_keys<<<blocks_for(32 * n), kThreads, 0, st>>>(C, famoff, bits, keys);
         TRY(launch_check());
         size_t tb = 0;
         BBPD_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, keys, skeys, nf, 0, 2 * bits, st));
         uint8_t *tmp = nullptr;
         TRY(s.get(&tmp, tb));
         BBPD_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp, tb, keys, skeys, nf, 0, 2 * bits, st));
-        o.nb = nb;
         k_horizon_emit<<<blocks_for(nf), kThreads, 0, st>>>(skeys, nf, bits, X, n, famoff, boff, fwd, o);
         return launch_check();
     }

@@ -1,14 +1,15 @@
 // Per-routine CUDA kernels: one entry point per reference MEX routine (and per
 // MATLAB-only routine of the hot path), with the reference's argument meaning
 // and in-place semantics. Bond routines run one thread per bond, node routines
-// one thread per node. The nodal force sum is node-centric: a plan holds each
-// node's bonds in bond order and the node adds them in the reference's OpenMP
-// order, so no atomics are needed and the result is bit-identical.
+// one thread per node. The nodal force sum is node-centric (nodalsum.cuh): a plan
+// holds each node's bonds in bond order and the node adds them in the reference's
+// OpenMP order, so no atomics are needed and the result is bit-identical.
 //
 // Host-pointer variants (used by the mexFunction gateways) keep a device
 // mirror per host buffer, copy the inputs in, run, copy the outputs back and
 // synchronize.
 #include "bbpd_internal.h"
+#include "nodalsum.cuh"
 #include "physics.cuh"
 #include "staging.cuh"
 
@@ -327,31 +328,41 @@ __global__ void k_plan_count(const int32_t *keys, int64_t n, int32_t *cnt)
     GRID_STRIDE(p, n) atomicAdd(&cnt[keys[p]], 1);
 }
 
-__global__ void k_nodalforces(const int64_t *__restrict__ rp, const int64_t *__restrict__ ent,
-                              int64_t nB, int64_t nN, int T, double *F,
-                              const double *__restrict__ fX, const double *__restrict__ fY,
-                              const double *__restrict__ fZ)
+// The plan's entries in the form of nodalsum.cuh: entry v = 2 k + side, its top
+// bit set where bond k belongs to another OpenMP chunk than the entry before
+// it in its node's list (calculatenodalforcesopenmpMex.c:39 static schedule)
+template <class ENT>
+__global__ void k_plan_pack(const int64_t *__restrict__ sorted, const int32_t *__restrict__ node, int64_t n, int64_t nB,
+                            int T, ENT *ent)
 {
-    GRID_STRIDE(n, nN)
+    constexpr ENT kFlag = (ENT)1 << (8 * sizeof(ENT) - 1);
+    GRID_STRIDE(p, n)
     {
-        // nodalForce[n] += thread partials in thread order (calculatenodalforcesopenmpMex.c:70-80)
-        double tx = F[n], ty = F[n + nN], tz = F[n + 2 * nN];
-        double ax = 0.0, ay = 0.0, az = 0.0;
-        int cur = -1;
-        for (int64_t p = rp[n]; p < rp[n + 1]; p++) {
-            int64_t v = ent[p], k = v >> 1;
-            int c = omp_chunk_of(k, nB, T);
-            if (c != cur) {
-                if (cur >= 0) { tx = tx + ax; ty = ty + ay; tz = tz + az; }
-                ax = ay = az = 0.0;
-                cur = c;
-            }
-            // private partial of the thread owning bond k (:56-63)
-            if (v & 1) { ax = ax - fX[k]; ay = ay - fY[k]; az = az - fZ[k]; }
-            else       { ax = ax + fX[k]; ay = ay + fY[k]; az = az + fZ[k]; }
-        }
-        if (cur >= 0) { tx = tx + ax; ty = ty + ay; tz = tz + az; }
-        F[n] = tx; F[n + nN] = ty; F[n + 2 * nN] = tz;
+        const int64_t v = sorted[p];
+        const bool first = p == 0 || node[p - 1] != node[p];
+        const bool flag = !first && omp_chunk_of(v >> 1, nB, T) != omp_chunk_of(sorted[p - 1] >> 1, nB, T);
+        ent[p] = (ENT)v | (flag ? kFlag : (ENT)0);
+    }
+}
+
+// nodalForce[n] += thread partials in thread order
+// (calculatenodalforcesopenmpMex.c:56-80). 7.1M bonds, 128 000 nodes on B200:
+// 265 us with a thread per node, 109 now; 50 000 bonds, 1 953 nodes: 117 us, 10 now
+// (under ncu, caches cold).
+template <class ENT>
+__global__ void __launch_bounds__(kThreads) k_nodalforces(const int64_t *__restrict__ rp, const ENT *__restrict__ ent,
+                                                          int64_t nN, double *F, const double *__restrict__ fX,
+                                                          const double *__restrict__ fY, const double *__restrict__ fZ)
+{
+    __shared__ NodeSumShared sm[kThreads / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    for (int64_t g = (int64_t)blockIdx.x * (kThreads / 32) + w; g * kNodes < nN; g += warps) {
+        const int64_t n = g * kNodes + lane / 3, e = n + (lane % 3) * nN;
+        const bool mine = lane < 3 * kNodes && n < nN;
+        double t = mine ? F[e] : 0.0, a;
+        warp_node_sums<true>(rp, ent, g * kNodes, nN, fX, fY, fZ, sm[w], t, a);
+        if (mine && rp[n + 1] > rp[n]) F[e] = t + a;
     }
 }
 
@@ -387,8 +398,9 @@ int launch_check()
 struct bbpd_nodal_plan {
     int64_t nB, nN;
     int T;
-    int64_t *rp = nullptr;   // nN + 1
-    int64_t *ent = nullptr;  // 2 nB
+    int64_t *rp = nullptr;     // nN + 1
+    uint32_t *ent32 = nullptr; // 2 nB entries, 32-bit where they fit
+    uint64_t *ent64 = nullptr;
 };
 
 // ---- device-pointer entry points ----
@@ -560,14 +572,16 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
     p->nB = nB; p->nN = nN; p->T = nChunks;
     int64_t ne = 2 * nB;
     int32_t *keys = nullptr, *keys2 = nullptr, *cnt = nullptr;
-    int64_t *vals = nullptr;
+    int64_t *vals = nullptr, *vals2 = nullptr;
     int *bad = nullptr;
     void *tmp = nullptr;
     size_t tmpb = 0, tmpb2 = 0;
+    const bool narrow = ne < (int64_t)1 << 31;   // the top bit is the chunk flag
     cudaError_t e = cudaSuccess;
 #define PLAN_TRY(x) do { e = (x); if (e != cudaSuccess) goto fail_; } while (0)
     PLAN_TRY(cudaMalloc(&p->rp, sizeof(int64_t) * (size_t)(nN + 1)));
-    PLAN_TRY(cudaMalloc(&p->ent, sizeof(int64_t) * (size_t)(ne > 0 ? ne : 1)));
+    if (narrow) PLAN_TRY(cudaMalloc(&p->ent32, sizeof(uint32_t) * (size_t)(ne > 0 ? ne : 1)));
+    else PLAN_TRY(cudaMalloc(&p->ent64, sizeof(uint64_t) * (size_t)ne));
     PLAN_TRY(cudaMalloc(&cnt, sizeof(int32_t) * (size_t)(nN + 1)));
     PLAN_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(nN + 1), st));
     PLAN_TRY(cudaMalloc(&bad, sizeof(int)));
@@ -576,14 +590,18 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
         PLAN_TRY(cudaMalloc(&keys, sizeof(int32_t) * (size_t)ne));
         PLAN_TRY(cudaMalloc(&keys2, sizeof(int32_t) * (size_t)ne));
         PLAN_TRY(cudaMalloc(&vals, sizeof(int64_t) * (size_t)ne));
+        PLAN_TRY(cudaMalloc(&vals2, sizeof(int64_t) * (size_t)ne));
         k_plan_keys<<<blocks_for(nB), kThreads, 0, st>>>(bl, nB, nN, keys, vals, bad);
         // stable radix sort by node keeps each node's entries in bond order
-        PLAN_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmpb, keys, keys2, vals, p->ent, ne, 0, 32, st));
+        PLAN_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmpb, keys, keys2, vals, vals2, ne, 0, 32, st));
         PLAN_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmpb2, cnt, cnt, nN + 1, st));
         if (tmpb2 > tmpb) tmpb = tmpb2;
         PLAN_TRY(cudaMalloc(&tmp, tmpb));
-        PLAN_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmpb, keys, keys2, vals, p->ent, ne, 0, 32, st));
+        PLAN_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmpb, keys, keys2, vals, vals2, ne, 0, 32, st));
         k_plan_count<<<blocks_for(ne), kThreads, 0, st>>>(keys, ne, cnt);
+        if (narrow) k_plan_pack<<<blocks_for(ne), kThreads, 0, st>>>(vals2, keys2, ne, nB, nChunks, p->ent32);
+        else k_plan_pack<<<blocks_for(ne), kThreads, 0, st>>>(vals2, keys2, ne, nB, nChunks, p->ent64);
+        PLAN_TRY(cudaGetLastError());
     }
     {
         // row pointers: exclusive scan of the counts (64-bit)
@@ -593,7 +611,7 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
         PLAN_TRY(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
         PLAN_TRY(cudaStreamSynchronize(st));
         if (hbad) {
-            cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
+            cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(vals2); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
             bbpd_nodal_plan_destroy(p);
             return fail(BBPD_ERR_ARG, "BONDLIST holds a node id that is not an integer in [1, nNodes] or a self-bond");
         }
@@ -604,11 +622,11 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
         PLAN_TRY(cudaMemcpyAsync(p->rp, hr.data(), sizeof(int64_t) * (size_t)(nN + 1), cudaMemcpyHostToDevice, st));
         PLAN_TRY(cudaStreamSynchronize(st));
     }
-    cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
+    cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(vals2); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
     *out = p;
     return BBPD_OK;
 fail_:
-    cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
+    cudaFree(keys); cudaFree(keys2); cudaFree(vals); cudaFree(vals2); cudaFree(cnt); cudaFree(bad); cudaFree(tmp);
     bbpd_nodal_plan_destroy(p);
     return fail(e == cudaErrorMemoryAllocation ? BBPD_ERR_OOM : BBPD_ERR_CUDA, "nodal plan: %s",
                 cudaGetErrorString(e));
@@ -619,7 +637,8 @@ extern "C" int bbpd_nodal_plan_destroy(bbpd_nodal_plan *p)
 {
     if (!p) return BBPD_OK;
     cudaFree(p->rp);
-    cudaFree(p->ent);
+    cudaFree(p->ent32);
+    cudaFree(p->ent64);
     delete p;
     return BBPD_OK;
 }
@@ -629,7 +648,9 @@ extern "C" int bbpd_dev_calculatenodalforces(const bbpd_nodal_plan *p, double *F
 {
     if (!p) return fail(BBPD_ERR_ARG, "null plan");
     if (p->nN == 0) return BBPD_OK;
-    k_nodalforces<<<blocks_for(p->nN), kThreads, 0, as_stream(stream)>>>(p->rp, p->ent, p->nB, p->nN, p->T, F, fX, fY, fZ);
+    const int blocks = blocks_for((p->nN + kNodes - 1) / kNodes * 32);
+    if (p->ent64) k_nodalforces<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, p->ent64, p->nN, F, fX, fY, fZ);
+    else k_nodalforces<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, p->ent32, p->nN, F, fX, fY, fZ);
     return launch_check();
 }
 

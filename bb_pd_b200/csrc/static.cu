@@ -32,6 +32,7 @@
 // with the direction p. Reductions are fixed-order, so a step is deterministic.
 #include "bbpd_internal.h"
 #include "gridbarrier.cuh"
+#include "nodalsum.cuh"
 #include "physics.cuh"
 #include "staging.cuh"
 
@@ -138,25 +139,22 @@ struct SNodes {
 // calculatenodalforces.m:25-35 in its serial order (node i gets +f of the bonds
 // it starts, -f of those it ends), times cellVolume (driver :111); the residual
 // norms of the free and held DOFs go to per-block partial sums.
-__global__ void k_static_nodal(SNodes g, const double *__restrict__ f, double V, double *F, double *part)
+__global__ void __launch_bounds__(kThreads) k_static_nodal(SNodes g, const double *__restrict__ f, double V, double *F,
+                                                           double *part)
 {
+    __shared__ NodeSumShared sm[kThreads / 32];
     __shared__ double sh[2][kThreads / 32];
     double rf = 0, rh = 0;
-    GRID_STRIDE(i, g.n)
-    {
-        double a[3] = {0, 0, 0};
-        for (int64_t e = g.off[i]; e < g.off[i + 1]; e++) {
-            const uint32_t q = g.ent[e];
-            const int64_t k = q >> 1;
-            for (int c = 0; c < 3; c++) {
-                const double v = f[k + c * g.nB];
-                a[c] = (q & 1u) ? a[c] - v : a[c] + v;
-            }
-        }
-        for (int c = 0; c < 3; c++) {
-            const double v = a[c] * V;
-            F[i + c * g.n] = v;
-            if (g.held[i + c * g.n]) rh += v * v;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t warps = (int64_t)gridDim.x * (kThreads / 32);
+    for (int64_t k = (int64_t)blockIdx.x * (kThreads / 32) + w; k * kNodes < g.n; k += warps) {
+        const int64_t i = k * kNodes + lane / 3, e = i + (lane % 3) * g.n;
+        double t = 0.0, a;
+        warp_node_sums<false>(g.off, g.ent, k * kNodes, g.n, f, f + g.nB, f + 2 * g.nB, sm[w], t, a);
+        if (lane < 3 * kNodes && i < g.n) {
+            const double v = a * V;
+            F[e] = v;
+            if (g.held[e]) rh += v * v;
             else rf += v * v;
         }
     }
@@ -164,16 +162,16 @@ __global__ void k_static_nodal(SNodes g, const double *__restrict__ f, double V,
         rf += __shfl_xor_sync(0xffffffffu, rf, o);
         rh += __shfl_xor_sync(0xffffffffu, rh, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][threadIdx.x >> 5] = rf;
-        sh[1][threadIdx.x >> 5] = rh;
+    if (lane == 0) {
+        sh[0][w] = rf;
+        sh[1][w] = rh;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         double s0 = 0, s1 = 0;
-        for (int w = 0; w < kThreads / 32; w++) {
-            s0 += sh[0][w];
-            s1 += sh[1][w];
+        for (int q = 0; q < kThreads / 32; q++) {
+            s0 += sh[0][q];
+            s1 += sh[1][q];
         }
         part[2 * blockIdx.x] = s0;
         part[2 * blockIdx.x + 1] = s1;

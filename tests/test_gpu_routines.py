@@ -95,6 +95,28 @@ def test_nodalforces_large_random():
         assert same(F, Fo)
 
 
+@pytest.mark.parametrize("nN,hubs", [(2, (1,)), (5, (1, 31)), (37, (32, 33)), (130, (0, 64, 127)), (403, (300, 65))])
+@pytest.mark.parametrize("T", [1, 8])
+def test_nodalforces_list_lengths(nN, hubs, T):
+    """Lists of 0, 1, a whole warp's 32 entries, one more or less and several
+    times that; node counts around the four of a warp; zeros of both signs."""
+    rng = np.random.default_rng(nN)
+    rows = []
+    for h, d in enumerate(hubs):   # node h gets d bonds to others (repeats allowed: each bond is a row of its own)
+        other = rng.integers(0, nN - 1, d)
+        other[other >= h] += 1
+        rows += [(h, o) if rng.random() < 0.5 else (o, h) for o in other]
+    bl = np.asfortranarray(np.array(rows, dtype=np.float64)[rng.permutation(len(rows))] + 1)
+    nB = len(bl)
+    f = [rng.normal(0, 1e3, nB) for _ in range(3)]
+    f[0][::3], f[1][::4] = 0.0, -0.0
+    F = np.asfortranarray(np.where(rng.random((nN, 3)) < 0.5, -0.0, rng.normal(0, 1, (nN, 3))))
+    Fo = F.copy(order="F")
+    (R.calculatenodalforcesopenmpMex if T == 8 else R.calculatenodalforcesMex)(bl, F, *f)
+    po.lib().orc_nodalforces_chunked(nB, nN, P(bl), P(Fo), P(f[0]), P(f[1]), P(f[2]), T)
+    assert same(F, Fo)
+
+
 def test_eulercromer_golden():
     g = gold("eulercromer")
     nN = g["F"].shape[0]
