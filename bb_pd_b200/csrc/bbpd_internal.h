@@ -33,6 +33,14 @@ namespace bbpd {
 // Fails with BBPD_ERR_NO_DEVICE when no CUDA device is visible: this library
 // has no CPU implementation to fall back to.
 int require_device();
+// Stream-ordered temporaries from a pool of the library's own on the current
+// device (freed with cudaFreeAsync). The default pool gives everything back to
+// the driver at each synchronisation, so a call that ends with one mapped its
+// temporaries anew every time; this pool keeps up to kScratchKeep bytes until
+// release_scratch (bbpd_release_mirrors) or process exit.
+constexpr uint64_t kScratchKeep = (uint64_t)256 << 20;
+cudaError_t scratch_malloc(void **p, size_t bytes, cudaStream_t st);
+void release_scratch();
 inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 }  // namespace bbpd
 #endif

@@ -71,7 +71,7 @@ struct Scratch {
     template <class T>
     int get(T **out, size_t count)
     {
-        BBPD_CUDA_TRY(cudaMallocAsync((void **)out, sizeof(T) * std::max<size_t>(count, 1), st));
+        BBPD_CUDA_TRY(scratch_malloc((void **)out, sizeof(T) * std::max<size_t>(count, 1), st));
         p.push_back((void *)*out);
         return BBPD_OK;
     }

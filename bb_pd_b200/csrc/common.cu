@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
+#include <vector>
 
 namespace bbpd {
 
@@ -30,6 +32,52 @@ int require_device()
                     e == cudaSuccess ? "count 0" : cudaGetErrorString(e));
     }
     return BBPD_OK;
+}
+
+namespace {
+std::mutex g_pool_mu;
+std::vector<cudaMemPool_t> g_pools;   // by device; null: not made (yet)
+}
+
+// The pool of device `dev`, made on first use; null where the device has none.
+static cudaMemPool_t scratch_pool(int dev)
+{
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if ((int)g_pools.size() <= dev) g_pools.resize(dev + 1, nullptr);
+    if (!g_pools[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t keep = kScratchKeep;
+        if (cudaMemPoolCreate(&g_pools[dev], &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(g_pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            g_pools[dev] = nullptr;
+        }
+    }
+    return g_pools[dev];
+}
+
+cudaError_t scratch_malloc(void **p, size_t bytes, cudaStream_t st)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (st && cudaStreamGetDevice(st, &dev) != cudaSuccess) cudaGetLastError();   // the stream's device, not the current one
+    if (cudaMemPool_t pool = scratch_pool(dev)) {
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+        if (e == cudaSuccess || e == cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();   // a pool that a device reset took away
+    }
+    return cudaMallocAsync(p, bytes, st);
+}
+
+void release_scratch()
+{
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    for (cudaMemPool_t p : g_pools)
+        if (p && cudaMemPoolTrimTo(p, 0) != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace bbpd

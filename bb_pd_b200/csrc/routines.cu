@@ -465,7 +465,7 @@ extern "C" int bbpd_dev_calculatedamage(const double *bl, const double *fail_, c
     if (rc) return rc;
     cudaStream_t st = as_stream(stream);
     int *bad = nullptr;
-    BBPD_CUDA_TRY(cudaMallocAsync(&bad, sizeof(int), st));
+    BBPD_CUDA_TRY(scratch_malloc((void **)&bad, sizeof(int), st));
     cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(damage, 0, sizeof(double) * (size_t)nN, st);
     if (e == cudaSuccess && nB > 0) {
@@ -543,7 +543,7 @@ extern "C" int bbpd_dev_calculatedampingcoefficient(const double *F, const doubl
     int64_t nsl = (nN + 31) / 32;
     const int64_t lv = 2 * ((nsl + 31) / 32) + 2;   // one level of the tree, both sums
     double *scratch = nullptr;   // 2 * nsl slice partials, 2 level buffers, 1 result
-    BBPD_CUDA_TRY(cudaMallocAsync(&scratch, sizeof(double) * (size_t)(2 * nsl + 2 * lv + 1), st));
+    BBPD_CUDA_TRY(scratch_malloc((void **)&scratch, sizeof(double) * (size_t)(2 * nsl + 2 * lv + 1), st));
     double *res = scratch + 2 * nsl + 2 * lv;
     if (nsl > 0)
         k_damping_slices<<<blocks_for(nsl * 32), kThreads, 0, st>>>(F, m, Fp, dt, vhp, u, nN, nsl, scratch);
@@ -720,6 +720,7 @@ extern "C" int bbpd_release_mirrors(void)
     g_mirrors.clear();
     if (g_plan.plan) bbpd_nodal_plan_destroy(g_plan.plan);
     g_plan = Plans{};
+    release_scratch();
     return BBPD_OK;
 }
 

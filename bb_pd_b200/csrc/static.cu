@@ -1140,7 +1140,7 @@ extern "C" int bbpd_dev_buildstiffnessmatrix(const double *X, int64_t nNodes, in
     CooBonds q{X, BONDLIST, VCF, BS, BFM, failFlag, BSF, n, nB, NOD, VOLUME};
     std::vector<void *> tmp;
     auto get = [&](void **p, size_t bytes) -> int {
-        BBPD_CUDA_TRY(cudaMallocAsync(p, std::max<size_t>(bytes, 8), st));
+        BBPD_CUDA_TRY(scratch_malloc(p, std::max<size_t>(bytes, 8), st));
         tmp.push_back(*p);
         return BBPD_OK;
     };
@@ -1240,7 +1240,7 @@ extern "C" int bbpd_buildstiffnessmatrix(const double *X, int64_t nNodes, int NO
         }
     } own{st, {}};
     auto up = [&](const double *h, int64_t cnt, double **d) -> int {
-        BBPD_CUDA_TRY(cudaMallocAsync((void **)d, sizeof(double) * std::max<int64_t>(cnt, 1), st));
+        BBPD_CUDA_TRY(scratch_malloc((void **)d, sizeof(double) * std::max<int64_t>(cnt, 1), st));
         own.p.push_back(*d);
         return h ? staging::upload_copy(*d, h, cnt, st) : BBPD_OK;
     };

@@ -309,8 +309,9 @@ int bbpd_buildmassmatrix(int64_t nNodes, double DX, double bondStiffnessConcrete
 int bbpd_dev_buildmassmatrix(int64_t nNodes, double DX, double bondStiffnessConcrete,
         double DT, const double *nFAMILYMEMBERS, double *massVector, void *stream);
 
-/* Free the device mirrors and cached plan of the host-pointer entry points
- * (the gateways register it with mexAtExit). */
+/* Free the device mirrors and cached plan of the host-pointer entry points, and
+ * the temporaries (at most 256 MB a device) that the builder and per-routine
+ * entry points keep between calls (the gateways register it with mexAtExit). */
 int bbpd_release_mirrors(void);
 
 /* replaces timeintegrationADR.m:1 (NOD = 3) */
