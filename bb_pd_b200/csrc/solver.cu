@@ -447,9 +447,44 @@ inline int quiet_high_word(double x)
     return (int)(b >> 32) & 0x7FFFFFFF;
 }
 
-// One entry in full generality: law, damage state written back when it
-// changes, bond force with the NaN guards of calculatebondforcesMex.c. Kept
-// out of line: intact bonds whose law is quiet never come here.
+// The law at stretch s of an entry whose state byte is sv and whose damage is
+// B0 (calculatebsf*.m / calculatebondfailureMex.c): the damage B and fail value
+// after it, with the state written back where it changed.
+template <int LAW>
+__device__ __forceinline__ void law_update(const Dev &d, int64_t e, int bt, uint32_t sv, double B0, double s, double scb,
+                                           double &B, double &failv)
+{
+    const LawScalars &P = d.P;
+    const double s0b = d.s0e ? __ldg(d.s0e + e) : P.s0;
+    const double s1b = d.s1e ? __ldg(d.s1e + e) : P.s1;
+    // damage-energy tracking: every step in which a concrete bond's stretch
+    // exceeds s0 comes here (the fast path requires s <= s0)
+    if (d.smax && bt == 0 && s > s0b && s > d.smax[e]) d.smax[e] = s;
+    B = B0;
+    bool soft = (sv & ST_SOFT) != 0;
+    failv = (sv & ST_BROKEN) ? 0.0 : 1.0;
+    const bool concrete = (bt == 0);
+    if (LAW == BBPD_LAW_TRILINEAR) {
+        law_trilinear(s, s0b, s1b, scb, P, d.s0e != nullptr || d.s1e != nullptr, concrete, B, soft);
+    } else if (LAW == BBPD_LAW_BILINEAR) {
+        law_bilinear(s, s0b, scb, concrete, B, soft);
+    } else if (LAW == BBPD_LAW_EXPONENTIAL) {
+        law_exponential(s, s0b, scb, P, concrete, B, soft);
+    } else {
+        law_linear(s, scb, P, bt, failv);
+    }
+    const bool dmg = __double_as_longlong(B) != 0;
+    // bits above the three state bits (the lattice form's BONDTYPE) are kept
+    const uint32_t stn = (soft ? ST_SOFT : 0u) | (failv == 0.0 ? ST_BROKEN : 0u) | (dmg ? ST_DAMAGED : 0u) |
+                         (sv & ~(uint32_t)ST_MASK);
+    if (stn != sv) d.st[e] = (uint8_t)stn;
+    if (__double_as_longlong(B) != __double_as_longlong(B0)) d.bsf[e] = B;
+}
+
+// One entry in full generality: IEEE kinematics, law, damage state written back
+// when it changes, bond force with the NaN guards of calculatebondforcesMex.c.
+// Bonds whose kinematics the branch-free pass cannot give come here, and in the
+// FP32 form those that need the law.
 #ifdef BBPD_GENERAL_OUTLINE
 #define BBPD_GENERAL_ATTR __noinline__
 #else
@@ -462,8 +497,6 @@ __device__ BBPD_GENERAL_ATTR double3 entry_general(const Dev &d, int64_t e, uint
 {
     const LawScalars &P = d.P;
     const int bt = (w >> BT_SHIFT) & 3;
-    const double s0b = d.s0e ? __ldg(d.s0e + e) : P.s0;
-    const double s1b = d.s1e ? __ldg(d.s1e + e) : P.s1;
     double dX, dY, dZ, L, s;
     float sf = 0.f, Lf = 0.f;
     bool exact = true;
@@ -486,30 +519,8 @@ __device__ BBPD_GENERAL_ATTR double3 entry_general(const Dev &d, int64_t e, uint
             L = (double)Lf;
         }
     }
-    // damage-energy tracking: every step in which a concrete bond's stretch
-    // exceeds s0 comes here (the fast path requires s <= s0)
-    if (d.smax && bt == 0 && s > s0b && s > d.smax[e]) d.smax[e] = s;
-    // law and damage (calculatebsf*.m / calculatebondfailureMex.c)
-    const double B0 = (sv & ST_DAMAGED) ? d.bsf[e] : 0.0;
-    double B = B0;
-    bool soft = (sv & ST_SOFT) != 0;
-    double failv = (sv & ST_BROKEN) ? 0.0 : 1.0;
-    const bool concrete = (bt == 0);
-    if (LAW == BBPD_LAW_TRILINEAR) {
-        law_trilinear(s, s0b, s1b, scb, P, d.s0e != nullptr || d.s1e != nullptr, concrete, B, soft);
-    } else if (LAW == BBPD_LAW_BILINEAR) {
-        law_bilinear(s, s0b, scb, concrete, B, soft);
-    } else if (LAW == BBPD_LAW_EXPONENTIAL) {
-        law_exponential(s, s0b, scb, P, concrete, B, soft);
-    } else {
-        law_linear(s, scb, P, bt, failv);
-    }
-    const bool dmg = __double_as_longlong(B) != 0;
-    // bits above the three state bits (the lattice form's BONDTYPE) are kept
-    const uint32_t stn = (soft ? ST_SOFT : 0u) | (failv == 0.0 ? ST_BROKEN : 0u) | (dmg ? ST_DAMAGED : 0u) |
-                         (sv & ~(uint32_t)ST_MASK);
-    if (stn != sv) d.st[e] = (uint8_t)stn;
-    if (__double_as_longlong(B) != __double_as_longlong(B0)) d.bsf[e] = B;
+    double B, failv;
+    law_update<LAW>(d, e, bt, sv, (sv & ST_DAMAGED) ? d.bsf[e] : 0.0, s, scb, B, failv);
     // bond force (calculatebondforcesMex.c:34-40)
     double3 f;
     if (PREC == kP64 || exact) {
@@ -570,60 +581,195 @@ __device__ __forceinline__ void load_pos(const double4 *p, double &x, double &y,
     (void)w;
 }
 
-// FP64 form, the fast path of one group of 4 entries of a lane at (xi, yi, zi):
-// without branches, so that the four dependency chains interleave. Returns the
-// mask of the slots that need the general path. Slots past the lane's list are
-// layout padding (all streams zero): they name node 0 and dictionary entry 0,
-// so every slot gathers a valid record and needs no select.
-template <int LAW, class CID, int SCE>
-__device__ __forceinline__ unsigned group_fast(const Dev &d, const Group<CID> &G, int64_t e0, bool safe,
-                                               const double4 *xa, double xi, double yi, double zi,
-                                               double (&fx)[4], double (&fy)[4], double (&fz)[4])
+// What the force of an entry needs of its neighbour and its bond.
+struct Rec {
+    double x, y, z;
+    DictEntry g;
+};
+
+__device__ __forceinline__ void load_rec(const Dev &d, const double4 *xa, uint32_t w, uint32_t c, Rec &r)
 {
-    double xj[4], yj[4], zj[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint32_t j = group_w(G, q) & COL_MASK;
-        load_pos(xa + j, xj[q], yj[q], zj[q]);
-    }
-    unsigned fast = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const uint32_t w = group_w(G, q);
-        const DictEntry g = ldg_dict(d.dict, G.cid(q));
-        const double dX = xj[q] - xi, dY = yj[q] - yi, dZ = zj[q] - zi;
-        double L, rL;
-        bool okr;
-        sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
-        const double s = quot_rn(L - g.l0, g.l0, g.rl0);
-        const double t = ((g.bs * s) * d.V) * g.vcf;
-        fx[q] = t * quot_rn(dX, L, rL);
-        fy[q] = t * quot_rn(dY, L, rL);
-        fz[q] = t * quot_rn(dZ, L, rL);
-        // tests on high words and without short circuits: no branch, no FP64
-        const bool intact = (G.s & (0xFFu << (8 * q))) == 0, regular = __double2hiint(g.rl0) >= 0;
-        bool quiet;
-        if (LAW == BBPD_LAW_LINEAR && SCE != 0) {
-            const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
-            quiet = law_quiet<LAW>(d.P, (w >> BT_SHIFT) & 3, s, 0.0, scv);
-        } else {
-            quiet = (__double2hiint(s) < d.quiet_hi) | (LAW != BBPD_LAW_LINEAR && (w & BT_BITS) != 0);
-        }
-        fast |= (okr & intact & regular & quiet ? 1u : 0u) << q;
-    }
-    return safe ? ~fast : ~0u;
+    load_pos(xa + (w & COL_MASK), r.x, r.y, r.z);
+    r.g = ldg_dict(d.dict, c);
 }
 
-// The general path of slot q of a group.
-template <int LAW, int PREC, class CID, int SCE>
-__device__ __forceinline__ double3 group_slow(const Dev &d, const Group<CID> &G, int q, int64_t e0, const double *xs,
-                                              double xi, double yi, double zi)
+// FP64 form, one entry of a lane at (xi, yi, zi), without a branch: its stretch
+// s, its direction (ux, uy, uz) = d / L and the scalar t of an intact bond's
+// force t u. `regular`: all of them are the reference's (the conditions of the
+// shared-divisor division hold); `fast`: the law is quiet and the bond intact too,
+// so t u is its force. The tests read high words and the group's state word gs,
+// without short circuits and without FP64 comparisons.
+template <int LAW, int SCE>
+__device__ __forceinline__ void entry_kinematics(const Dev &d, const Rec &r, uint32_t w, uint32_t gs, int q, int64_t e,
+                                                 double xi, double yi, double zi, double &s, double &t, double &ux,
+                                                 double &uy, double &uz, bool &regular, bool &fast)
 {
-    const int64_t nN = d.n_nodes;
-    const uint32_t w = group_w(G, q), j = w & COL_MASK;
-    const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e0 + q) : d.P.sc;
-    return entry_general<LAW, PREC>(d, e0 + q, w, (G.s >> (8 * q)) & 0xFFu, ldg_dict(d.dict, G.cid(q)), scv, xi, yi,
-                                    zi, xs[j], xs[j + nN], xs[j + 2 * nN]);
+    const double dX = r.x - xi, dY = r.y - yi, dZ = r.z - zi;
+    double L, rL;
+    bool okr;
+    sqrt_recip_rn(dX * dX + dY * dY + dZ * dZ, L, rL, okr);
+    s = quot_rn(L - r.g.l0, r.g.l0, r.g.rl0);
+    t = ((r.g.bs * s) * d.V) * r.g.vcf;
+    ux = quot_rn(dX, L, rL);
+    uy = quot_rn(dY, L, rL);
+    uz = quot_rn(dZ, L, rL);
+    const bool intact = (gs & (0xFFu << (8 * q))) == 0;
+    bool quiet;
+    if (LAW == BBPD_LAW_LINEAR && SCE != 0) {
+        const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e) : d.P.sc;
+        quiet = law_quiet<LAW>(d.P, (w >> BT_SHIFT) & 3, s, 0.0, scv);
+    } else {
+        quiet = (__double2hiint(s) < d.quiet_hi) | (LAW != BBPD_LAW_LINEAR && (w & BT_BITS) != 0);
+    }
+    regular = okr & (__double2hiint(r.g.rl0) >= 0);
+    fast = regular & intact & quiet;
+}
+
+// Force of one entry whose streams are not in registers, whatever its state.
+template <int LAW, int PREC, class CID, int SCE>
+__device__ __forceinline__ double3 entry_careful(const Dev &d, int64_t e, uint32_t w, bool safe, const double4 *xa,
+                                                 double xi, double yi, double zi)
+{
+    const uint32_t sv = d.st[e];
+    const double B0 = (sv & ST_DAMAGED) ? d.bsf[e] : 0.0;
+    Rec r;
+    load_rec(d, xa, w, reinterpret_cast<const CID *>(d.cid)[e], r);
+    double s, t;
+    double3 f;
+    bool regular, fast;
+    entry_kinematics<LAW, SCE>(d, r, w, sv, 0, e, xi, yi, zi, s, t, f.x, f.y, f.z, regular, fast);
+    if (!(fast & safe)) {
+        const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e) : d.P.sc;
+        if (!(regular & safe)) return entry_general<LAW, PREC>(d, e, w, sv, r.g, scv, xi, yi, zi, r.x, r.y, r.z);
+        double B, failv;
+        law_update<LAW>(d, e, (w >> BT_SHIFT) & 3, sv, B0, s, scv, B, failv);
+        t = bond_force_scalar(failv, r.g.bs, B, s, 0.0, d.V, r.g.vcf);
+    }
+    f.x = t * f.x;
+    f.y = t * f.y;
+    f.z = t * f.z;
+    if (f.x != f.x) f.x = 0.0;   // calculatebondforcesMex.c:37-40
+    if (f.y != f.y) f.y = 0.0;
+    if (f.z != f.z) f.z = 0.0;
+    return f;
+}
+
+// Forces of the first nq entries of a group, whatever their state; the others
+// give -0, which leaves every sum as it is. Slots past the lane's list are
+// layout padding (all streams zero): they name node 0 and dictionary entry 0,
+// so every slot gathers a valid record. Entries of damaged, broken or softening
+// bonds keep the stretch and direction of the branch-free pass and only run the
+// law. The damage of the four entries lies side by side and is read before the
+// pass. Past its peak the 20 000-node beam takes 49 us a step so, 56 with
+// entry_careful for every such bond, 65 with IEEE kinematics for each.
+template <int LAW, int PREC, class CID, int SCE>
+__device__ __forceinline__ void group_forces(const Dev &d, const Group<CID> &G, int64_t e0, int nq, bool safe,
+                                             const double4 *xa, double xi, double yi, double zi, double (&fx)[4],
+                                             double (&fy)[4], double (&fz)[4])
+{
+    Rec r[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) load_rec(d, xa, group_w(G, q), G.cid(q), r[q]);
+    double B0[4] = {0.0, 0.0, 0.0, 0.0};
+    if (G.s & (0x01010101u * ST_DAMAGED))
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(B0[0]), "=d"(B0[1]), "=d"(B0[2]), "=d"(B0[3])
+                     : "l"(d.bsf + e0));
+    double s[4], t[4];
+    unsigned slow = 0, reg = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        bool regular, fast;
+        entry_kinematics<LAW, SCE>(d, r[q], group_w(G, q), G.s, q, e0 + q, xi, yi, zi, s[q], t[q], fx[q], fy[q], fz[q],
+                                   regular, fast);
+        slow |= (fast & safe ? 0u : 1u) << q;
+        reg |= (regular & safe ? 1u : 0u) << q;
+    }
+    slow &= (1u << nq) - 1;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if (slow & (1u << q)) {
+            const int64_t e = e0 + q;
+            const uint32_t w = group_w(G, q), sv = (G.s >> (8 * q)) & 0xFFu;
+            const DictEntry g = ldg_dict(d.dict, G.cid(q));
+            const double scv = has_sce<SCE>(d) ? __ldcs(d.sce + e) : d.P.sc;
+            if (reg & (1u << q)) {
+                double B, failv;
+                law_update<LAW>(d, e, (w >> BT_SHIFT) & 3, sv, (sv & ST_DAMAGED) ? B0[q] : 0.0, s[q], scv, B, failv);
+                t[q] = bond_force_scalar(failv, g.bs, B, s[q], 0.0, d.V, g.vcf);
+                fx[q] = t[q] * fx[q];
+                fy[q] = t[q] * fy[q];
+                fz[q] = t[q] * fz[q];
+                if (fx[q] != fx[q]) fx[q] = 0.0;
+                if (fy[q] != fy[q]) fy[q] = 0.0;
+                if (fz[q] != fz[q]) fz[q] = 0.0;
+            } else {
+                double x, y, z;
+                load_pos(xa + (w & COL_MASK), x, y, z);
+                const double3 f = entry_general<LAW, PREC>(d, e, w, sv, g, scv, xi, yi, zi, x, y, z);
+                fx[q] = f.x;
+                fy[q] = f.y;
+                fz[q] = f.z;
+            }
+        } else {
+            fx[q] = q < nq ? t[q] * fx[q] : -0.0;
+            fy[q] = q < nq ? t[q] * fy[q] : -0.0;
+            fz[q] = q < nq ? t[q] * fz[q] : -0.0;
+        }
+    }
+}
+
+// The same where every bond of the warp's groups is intact and quiet: true then,
+// and false where group_forces has to be called (before any work where the
+// state words tell).
+template <int LAW, class CID, int SCE>
+__device__ __forceinline__ bool group_fast(const Dev &d, const Group<CID> &G, int64_t e0, int nq, bool safe,
+                                           const double4 *xa, double xi, double yi, double zi, double (&fx)[4],
+                                           double (&fy)[4], double (&fz)[4])
+{
+    if (__any_sync(0xffffffffu, G.s != 0) || !safe) return false;
+    Rec r[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) load_rec(d, xa, group_w(G, q), G.cid(q), r[q]);
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        double s, t;
+        bool regular, fast;
+        entry_kinematics<LAW, SCE>(d, r[q], group_w(G, q), 0u, q, e0 + q, xi, yi, zi, s, t, fx[q], fy[q], fz[q], regular,
+                                   fast);
+        fx[q] = q < nq ? t * fx[q] : -0.0;
+        fy[q] = q < nq ? t * fy[q] : -0.0;
+        fz[q] = q < nq ? t * fz[q] : -0.0;
+        ok &= fast | (q >= nq);
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+// The fast path of one group of 4 entries of a lane, without branches, so that
+// the four dependency chains interleave: the forces of intact bonds whose law is
+// quiet, and the mask of the slots that need entry_careful.
+template <int LAW, class CID, int SCE>
+__device__ __forceinline__ unsigned group_pass(const Dev &d, const Group<CID> &G, int64_t e0, bool safe,
+                                               const double4 *xa, double xi, double yi, double zi, double (&fx)[4],
+                                               double (&fy)[4], double (&fz)[4])
+{
+    Rec r[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) load_rec(d, xa, group_w(G, q), G.cid(q), r[q]);
+    unsigned ok = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        double s, t;
+        bool regular, fast;
+        entry_kinematics<LAW, SCE>(d, r[q], group_w(G, q), G.s, q, e0 + q, xi, yi, zi, s, t, fx[q], fy[q], fz[q], regular,
+                                   fast);
+        fx[q] = t * fx[q];
+        fy[q] = t * fy[q];
+        fz[q] = t * fz[q];
+        ok |= (fast ? 1u : 0u) << q;
+    }
+    return safe ? ~ok : ~0u;
 }
 
 // Forces of the 32 nodes of one slice (FP64 form).
@@ -633,8 +779,7 @@ __device__ __forceinline__ double3 group_slow(const Dev &d, const Group<CID> &G,
 // node's force summed in the reference's order.
 template <int LAW, int PREC, class CID, int SCE>
 __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane, bool safe,
-                                             const double *xs, const double4 *xa, double &tx, double &ty,
-                                             double &tz)
+                                             const double4 *xa, double &tx, double &ty, double &tz)
 {
     const int64_t nN = d.n_nodes;
     const int64_t i = sl * 32 + lane;
@@ -642,7 +787,7 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
     const int64_t sb = d.slice_ptr[sl];
 
     double xi = 0, yi = 0, zi = 0;
-    if (i < nN) { xi = xs[i]; yi = xs[i + nN]; zi = xs[i + 2 * nN]; }
+    if (i < nN) load_pos(xa + i, xi, yi, zi);
     tx = 0.0; ty = 0.0; tz = 0.0;
     double ax = 0.0, ay = 0.0, az = 0.0;
 
@@ -655,7 +800,7 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
         if (g + 1 < ng) load_group<CID>(d, e0 + 128, Gn);
         const int nq = min(4, dg - 4 * g);
         double fx[4], fy[4], fz[4];
-        const unsigned slow = group_fast<LAW, CID, SCE>(d, Gc, e0, safe, xa, xi, yi, zi, fx, fy, fz) & ((1u << nq) - 1);
+        const unsigned slow = group_pass<LAW, CID, SCE>(d, Gc, e0, safe, xa, xi, yi, zi, fx, fy, fz) & ((1u << nq) - 1);
         // the sum in the reference's order: a full group with no general entry
         // and no chunk start (nearly every group) adds its four forces
         // straight; otherwise each entry is taken in turn
@@ -666,16 +811,21 @@ __device__ __forceinline__ void slice_forces(const Dev &d, int64_t sl, int lane,
             Gc = Gn;
             continue;
         }
+        for (unsigned left = slow; left; left &= left - 1) {   // lanes take their slow slots side by side
+            const int q = __ffs(left) - 1;
+            const double3 r = entry_careful<LAW, PREC, CID, SCE>(d, e0 + q, group_w(Gc, q), safe, xa, xi, yi, zi);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (k == q) { fx[k] = r.x; fy[k] = r.y; fz[k] = r.z; }
+        }
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             if (q < nq) {
-                double3 r = make_double3(fx[q], fy[q], fz[q]);
-                if (slow & (1u << q)) r = group_slow<LAW, PREC, CID, SCE>(d, Gc, q, e0, xs, xi, yi, zi);
                 if (group_w(Gc, q) & F_CHUNK) {  // partial of the previous OpenMP thread is complete
                     tx = tx + ax; ty = ty + ay; tz = tz + az;
                     ax = 0.0; ay = 0.0; az = 0.0;
                 }
-                ax = ax + r.x; ay = ay + r.y; az = az + r.z;
+                ax = ax + fx[q]; ay = ay + fy[q]; az = az + fz[q];
             }
         }
         Gc = Gn;
@@ -1145,7 +1295,7 @@ __global__ void __launch_bounds__(kBlock, PREC == kP32X ? BBPD_MIN_BLOCKS_F32 : 
             if (PREC != kP32X) prefetch_slice_head<CID, SCE>(d, sl_next, lane);
             double tx, ty, tz;
             if (PREC == kP32X) slice_forces_x<LAW, CID, SCE, false>(d, sl, lane, b.xs, b.urhs, b.urls, tx, ty, tz);
-            else slice_forces<LAW, PREC, CID, SCE>(d, sl, lane, safe, b.xs, b.xas, tx, ty, tz);
+            else slice_forces<LAW, PREC, CID, SCE>(d, sl, lane, safe, b.xas, tx, ty, tz);
             finish_slice<SCHEME, PREC>(d, b, sl, lane, tx, ty, tz, it);
             sl = sl_next;
         }
@@ -1281,28 +1431,24 @@ __global__ void __launch_bounds__(kSplitBlock, 1) split_kernel(Dev d, int64_t st
                     if (g + nteam < G1) load_group<CID>(d, e0 + 128 * nteam, Gn);
                     const int nq = max(0, min(4, dg - 4 * g));
                     double fx[4], fy[4], fz[4];
-                    unsigned slow;
+                    unsigned slow = 0;   // FP32 form: slots that take the general path below
                     if (PREC == kP32X) {
                         float gx[4], gy[4], gz[4];
                         slow = group_fast_x<LAW, CID, SCE>(d, Gc, e0, b.urhs, b.urls, ui, li, gx, gy, gz);
 #pragma unroll
                         for (int q = 0; q < 4; q++) { fx[q] = (double)gx[q]; fy[q] = (double)gy[q]; fz[q] = (double)gz[q]; }
-                    } else {
-                        slow = group_fast<LAW, CID, SCE>(d, Gc, e0, safe, b.xas, xi, yi, zi, fx, fy, fz);
+                    } else if (!group_fast<LAW, CID, SCE>(d, Gc, e0, nq, safe, b.xas, xi, yi, zi, fx, fy, fz)) {
+                        group_forces<LAW, PREC, CID, SCE>(d, Gc, e0, nq, safe, b.xas, xi, yi, zi, fx, fy, fz);
                     }
                     unsigned cb = 0;
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         double3 r = make_double3(fx[q], fy[q], fz[q]);
-                        if (q >= nq) {
-                            r = make_double3(-0.0, -0.0, -0.0);   // x + -0 is x, whatever x
-                        } else {
-                            if (slow & (1u << q)) {
-                                if (PREC == kP32X) r = group_slow_x<LAW, CID, SCE>(d, Gc, q, e0, i, b.xs);
-                                else r = group_slow<LAW, PREC, CID, SCE>(d, Gc, q, e0, b.xs, xi, yi, zi);
-                            }
-                            if (group_w(Gc, q) & F_CHUNK) cb |= 1u << q;
+                        if (PREC == kP32X) {
+                            if (q >= nq) r = make_double3(-0.0, -0.0, -0.0);   // x + -0 is x, whatever x
+                            else if (slow & (1u << q)) r = group_slow_x<LAW, CID, SCE>(d, Gc, q, e0, i, b.xs);
                         }
+                        if (q < nq && (group_w(Gc, q) & F_CHUNK)) cb |= 1u << q;
                         double *f = sF + (4 * (g - G0) + q) * 32 + lane;
                         f[0] = r.x;
                         f[kC] = r.y;
@@ -1957,7 +2103,7 @@ __global__ void __launch_bounds__(kBlock, BBPD_MIN_BLOCKS) batch_kernel(BatchCtl
                 const bool safe = (*(volatile unsigned *)d.sticky & 1u) == 0;
                 double tx, ty, tz;
                 if (PREC == kP32X) slice_forces_x<LAW, uint16_t, SCE, true>(d, sl, lane, b.xs, b.urhs, b.urls, tx, ty, tz);
-                else slice_forces<LAW, PREC, uint16_t, SCE>(d, sl, lane, safe, b.xs, b.xas, tx, ty, tz);
+                else slice_forces<LAW, PREC, uint16_t, SCE>(d, sl, lane, safe, b.xas, tx, ty, tz);
                 finish_slice<BBPD_SCHEME_ADR, PREC>(d, b, sl, lane, tx, ty, tz, it);
             }
             gi = gnext;
@@ -1988,7 +2134,7 @@ __device__ __noinline__ void mixed_law_slice(const Dev &d, const StepBufs &b, in
     const bool safe = (*(volatile unsigned *)d.sticky & 1u) == 0;
     double tx, ty, tz;
     if (PREC == kP32X) slice_forces_x<LAW, uint16_t, 2, true>(d, sl, lane, b.xs, b.urhs, b.urls, tx, ty, tz);
-    else slice_forces<LAW, PREC, uint16_t, 2>(d, sl, lane, safe, b.xs, b.xas, tx, ty, tz);
+    else slice_forces<LAW, PREC, uint16_t, 2>(d, sl, lane, safe, b.xas, tx, ty, tz);
     finish_slice<BBPD_SCHEME_ADR, PREC>(d, b, sl, lane, tx, ty, tz, it);
 }
 
