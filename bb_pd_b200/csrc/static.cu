@@ -217,18 +217,6 @@ __global__ void k_slice_fill(const int64_t *__restrict__ off, const uint32_t *__
     }
 }
 
-// Segments of every slice: warp w sums rows [w chunk, (w + 1) chunk), and its
-// part of slice s is segment s + w
-__global__ void k_segments(const int64_t *__restrict__ sptr, int64_t ns, int64_t chunk, int32_t *seg)
-{
-    GRID_STRIDE(s, ns)
-    {
-        const int64_t a = sptr[s] >> 5, b = sptr[s + 1] >> 5;
-        seg[2 * s] = (int32_t)(s + a / chunk);
-        seg[2 * s + 1] = b > a ? (int32_t)(s + (b - 1) / chunk + 1) : seg[2 * s];
-    }
-}
-
 // A node's position and its component of the CG direction p (zero on held and
 // left-out DOFs): 64 bytes, read as a 256-bit and a 128-bit load
 struct __align__(64) NodeRec {
@@ -270,29 +258,26 @@ __global__ void k_slot_rig(const uint32_t *__restrict__ bond, const double *__re
     }
 }
 
-__global__ void k_static_precond(SNodes g, const double *__restrict__ rig, const NodeRec *__restrict__ rec, double *Minv,
+// A lane adds its node's list in bond order, four rows of the slice in flight.
+__global__ void k_static_precond(SNodes g, const double *__restrict__ rigE, const NodeRec *__restrict__ rec, double *Minv,
                                  uint8_t *skip)
 {
     const int64_t n = g.n;
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    GRID_STRIDE(i, n)
+    {
+        const int64_t s = i >> 5, rows = (g.sptr[s + 1] - g.sptr[s]) >> 5;
+        const uint32_t *col = g.col + g.sptr[s] + (i & 31);
+        const double *rig = rigE + g.sptr[s] + (i & 31);
         const double xi[3] = {rec[i].x, rec[i].y, rec[i].z};
-        double S[6] = {0, 0, 0, 0, 0, 0};   // D00 D01 D02 D11 D12 D22
-        for (int64_t e = g.off[i] + lane; e < g.off[i + 1]; e += 32) {
-            const uint32_t q = g.ent[e];
-            const double r = rig[q >> 1];
-            if (r == 0) continue;
-            const NodeRec *o = rec + ((q & 1u) ? g.a[q >> 1] : g.b[q >> 1]);
+        double D[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+#pragma unroll 4
+        for (int64_t k = 0; k < rows; k++) {
+            const double r = rig[k * 32];
+            const NodeRec *o = rec + col[k * 32];
             const double c[3] = {o->x - xi[0], o->y - xi[1], o->z - xi[2]};
-            int k = 0;
             for (int u = 0; u < 3; u++)
-                for (int v = u; v < 3; v++) S[k++] += r * c[u] * c[v];
+                for (int v = 0; v < 3; v++) D[u][v] += r != 0 ? r * c[u] * c[v] : 0.0;
         }
-        for (int o = 16; o > 0; o >>= 1)
-            for (int q = 0; q < 6; q++) S[q] += __shfl_xor_sync(0xffffffffu, S[q], o);
-        if (lane != 0) continue;
-        double D[3][3] = {{S[0], S[1], S[2]}, {S[1], S[3], S[4]}, {S[2], S[4], S[5]}};
         bool fr[3];
         for (int u = 0; u < 3; u++) {
             fr[u] = !g.held[i + u * n] && D[u][u] > 0;
@@ -344,49 +329,46 @@ __global__ void k_reduce(const double *__restrict__ part, int nb, int w, double 
     if (lane == 0) out[k] = s;
 }
 
-// Two sums over the block's threads, in a fixed order (every thread gets them)
-__device__ __forceinline__ void block_sum2(double &u, double &v, double (*sh)[32])
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        u += __shfl_xor_sync(0xffffffffu, u, o);
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    __syncthreads();   // sh is free
-    if (lane == 0) {
-        sh[0][w] = u;
-        sh[1][w] = v;
-    }
-    __syncthreads();
-    u = lane < nw ? sh[0][lane] : 0.0;
-    v = lane < nw ? sh[1][lane] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) {
-        u += __shfl_xor_sync(0xffffffffu, u, o);
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-}
-
-// The grid's two sums: every block publishes its own and, after the barrier,
-// adds all of them for itself in the same order.
-__device__ __forceinline__ bool grid_sum2(double &u, double &v, double (*sh)[32], double2 *part, GridBarrier &bar)
-{
-    block_sum2(u, v, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = make_double2(u, v);
-    if (!bar.wait()) return false;
-    u = v = 0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
-        const double2 p = __ldcg(&part[k]);
-        u += p.x;
-        v += p.y;
-    }
-    block_sum2(u, v, sh);
-    return true;
-}
-
 constexpr int kCgThreads = 512;   // 16 warps of 128 registers on every SM
+constexpr int kCgWarps = kCgThreads / 32;
 constexpr int kCgRows = 4;         // rows of a warp's gathers in flight
 constexpr int kCgCheck = 8;        // iterations between convergence checks
 constexpr int kCgLaunch = 1024;    // iterations of one launch at most
+// The sums keep the order of 592 groups of 8 warps, whatever the grid: p.Kp goes
+// over the nodes warp by warp (lane l of owner o stands for warp 32 o + l, which
+// takes nodes 32 o + l, 32 o + l + 4736, ...), r.z and r.r over them 32 at a time.
+constexpr int kCgGroups = 592;
+constexpr int kCgOwners = kCgGroups / 4;
+constexpr int kCgSlices = 5;       // slices a block multiplies between two syncs: 15 sums for its 16 warps
+
+struct CgShared {
+    double acc[kCgSlices][kCgWarps][3][32];   // K p: two of a node's 32 partial sums, folded
+    double py[kCgSlices][3][32];              // p_c (K p)_c
+    double2 part[kCgGroups];
+    double sh[2][kCgWarps];
+    double2 sum;
+};
+
+// The grid's two sums: every block adds the groups' partials for itself, in
+// group order, after the barrier.
+__device__ __forceinline__ double2 add_groups(const double2 *part, int count, CgShared &sm)
+{
+    for (int k = threadIdx.x; k < count; k += kCgThreads) sm.part[k] = __ldcg(&part[k]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double u = 0;
+#pragma unroll 8
+        for (int k = 0; k < count; k++) u += sm.part[k].x;
+        sm.sum.x = u;
+    } else if (threadIdx.x == 32) {
+        double v = 0;
+#pragma unroll 8
+        for (int k = 0; k < count; k++) v += sm.part[k].y;
+        sm.sum.y = v;
+    }
+    __syncthreads();
+    return sm.sum;
+}
 
 struct CgArgs {
     SNodes g;
@@ -396,58 +378,186 @@ struct CgArgs {
     const uint8_t *skip;
     double *x;                     // moved by the solution once the solve ends
     double *d, *r, *z;
-    double *yseg;                  // partial K p of every segment: [segment][component][lane]
-    const int32_t *seg;            // segments of slice s: [seg[2 s], seg[2 s + 1])
-    double2 *part;                 // 2 x gridDim block partials
+    double *y;                     // K p
+    double2 *part;                 // 2 x kCgGroups partials
     double *scal;                  // [0] r.z, [1] r.r, [2] r.r at the start
     int *state;                    // [0] CG_*, [1] iterations so far, [2] error word
     unsigned *bar;
     unsigned long long timeout_ns;
     double tol2;                   // stop at r.r <= tol2 * r.r at the start
     int first, max_cg;
-    int64_t rows;                  // rows of 32 slots, all slices together
-    int64_t chunk;                 // consecutive rows of one warp
 };
 enum { CG_MORE = 0, CG_DONE = 1, CG_NONFINITE = 2 };
+
+// r.z and r.r of all nodes: node(i, rz, rr) does a node's work and adds its terms.
+// A warp takes 32 nodes, 8 warps a group; sums over the warp, then the group.
+template <class F>
+__device__ __forceinline__ void node_sums(int64_t n, double2 *part, CgShared &sm, F node)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int groups = (int)min((int64_t)kCgGroups, (n + 255) / 256);
+    for (int v0 = 0; v0 < groups; v0 += 2 * gridDim.x) {
+        const int v = v0 + blockIdx.x + (w >> 3) * gridDim.x;
+        double rz = 0, rr = 0;
+        if (v < groups)
+            for (int64_t i = 256 * (int64_t)v + 32 * (w & 7) + lane; i < n; i += 256 * (int64_t)kCgGroups) node(i, rz, rr);
+        for (int o = 16; o > 0; o >>= 1) {
+            rz += __shfl_xor_sync(0xffffffffu, rz, o);
+            rr += __shfl_xor_sync(0xffffffffu, rr, o);
+        }
+        __syncthreads();   // sh is free
+        if (lane == 0) {
+            sm.sh[0][w] = rz;
+            sm.sh[1][w] = rr;
+        }
+        __syncthreads();
+        if ((threadIdx.x & 255) == 0 && v < groups) {
+            double2 s = make_double2(0, 0);
+            for (int k = 0; k < 8; k++) {
+                s.x += sm.sh[0][w + k];
+                s.y += sm.sh[1][w + k];
+            }
+            part[v] = s;
+        }
+    }
+}
+
+// y = K p of the owners' slices (slice s belongs to owner s mod kCgOwners) and the
+// partials of p.y. A node's sum is 32 partial sums (entries l, l + 32, ... to
+// partial l) folded in a butterfly; warp w of the block takes partials w and
+// w + 16 of the slice's 32 nodes.
+__device__ __forceinline__ void cg_product(const SNodes &g, const double *rigE, const NodeRec *rec, double *y, double2 *part,
+                                           CgShared &sm)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t n = g.n;
+    for (int own = blockIdx.x; own < kCgOwners && own < g.ns; own += gridDim.x) {
+        const int64_t count = (g.ns - own + kCgOwners - 1) / kCgOwners;
+        double acc = 0;   // warp 0: p.y of the warp this lane stands for
+        for (int64_t m = 0; m < count; m += kCgSlices) {
+            const int G = (int)min((int64_t)kCgSlices, count - m);
+            // lane k < G holds the place and rows of slice k
+            int64_t at = 0;
+            int len = 0;
+            if (lane < G) {
+                const int64_t s = own + kCgOwners * (m + lane);
+                at = g.sptr[s];
+                len = (int)((g.sptr[s + 1] - at) >> 5);
+            }
+            uint32_t j[kCgRows];
+            double h[kCgRows];
+            // rows k, k + 32, ... of slice q, if it has them: neighbours and scales
+            auto streams = [&](int q, int k) {
+                const int64_t b = __shfl_sync(0xffffffffu, at, q) + lane;
+                const int rows = __shfl_sync(0xffffffffu, len, q);
+#pragma unroll
+                for (int t = 0; t < kCgRows; t++) {
+                    const int row = k + 32 * t;
+                    j[t] = row < rows ? __ldg(g.col + b + (int64_t)row * 32) : 0u;
+                    h[t] = row < rows ? __ldg(rigE + b + (int64_t)row * 32) : 0.0;
+                }
+            };
+            streams(0, w);
+            for (int q = 0; q < G; q++) {
+                const int64_t i = (own + kCgOwners * (m + q)) * 32 + lane;
+                const int rows = __shfl_sync(0xffffffffu, len, q);
+                Rec6 o = {0, 0, 0, 0, 0, 0};
+                if (i < n) o = load_rec(rec + i);
+                double u0 = 0, u1 = 0, u2 = 0;
+                for (int half = 0; half < 2; half++) {
+                    double y0 = 0, y1 = 0, y2 = 0;
+                    for (int k = w + 16 * half;;) {
+                        Rec6 v[kCgRows];
+                        double r[kCgRows];
+#pragma unroll
+                        for (int t = 0; t < kCgRows; t++) {
+                            v[t] = load_rec(rec + j[t]);
+                            r[t] = h[t];
+                        }
+                        k += 32 * kCgRows;
+                        const bool more = k < rows;
+                        if (more) streams(q, k);
+                        else if (half == 0) streams(q, w + 16);
+                        else if (q + 1 < G) streams(q + 1, w);
+#pragma unroll
+                        for (int t = 0; t < kCgRows; t++) {
+                            const double c0 = v[t].x - o.x, c1 = v[t].y - o.y, c2 = v[t].z - o.z;
+                            const double e = r[t] * (c0 * (o.px - v[t].px) + c1 * (o.py - v[t].py) + c2 * (o.pz - v[t].pz));
+                            // a failed bond (scale 0) adds nothing, whatever its ends hold
+                            y0 += r[t] != 0 ? e * c0 : 0.0;
+                            y1 += r[t] != 0 ? e * c1 : 0.0;
+                            y2 += r[t] != 0 ? e * c2 : 0.0;
+                        }
+                        if (!more) break;
+                    }
+                    u0 = half ? u0 + y0 : y0;
+                    u1 = half ? u1 + y1 : y1;
+                    u2 = half ? u2 + y2 : y2;
+                }
+                sm.acc[q][w][0][lane] = u0;
+                sm.acc[q][w][1][lane] = u1;
+                sm.acc[q][w][2][lane] = u2;
+            }
+            __syncthreads();
+            for (int f = w; f < 3 * G; f += kCgWarps) {
+                const int q = f / 3, c = f % 3;
+                const int64_t i = (own + kCgOwners * (m + q)) * 32 + lane;
+                double t[kCgWarps];
+#pragma unroll
+                for (int k = 0; k < kCgWarps; k++) t[k] = sm.acc[q][k][c][lane];
+#pragma unroll
+                for (int d = kCgWarps / 2; d > 0; d >>= 1)
+#pragma unroll
+                    for (int k = 0; k < d; k++) t[k] += t[k + d];
+                if (i < n) {
+                    const double v = g.held[i + c * n] ? 0.0 : t[0];
+                    y[i + c * n] = v;
+                    sm.py[q][c][lane] = (&rec[i].px)[c] * v;
+                }
+            }
+            __syncthreads();
+            if (w == 0)
+                for (int q = 0; q < G; q++)
+                    if ((own + kCgOwners * (m + q)) * 32 + lane < n)
+                        for (int c = 0; c < 3; c++) acc += sm.py[q][c][lane];
+        }
+        if (w == 0) {
+            double s = 0;
+            for (int k = 0; k < 8; k++) s += __shfl_sync(0xffffffffu, acc, (lane & 3) * 8 + k);
+            if (lane < 4) part[4 * own + lane] = make_double2(s, 0.0);
+        }
+    }
+}
 
 // The linear solve K delta = F on the free DOFs by conjugate gradients, one
 // persistent launch: three barriers an iteration (after p.Kp, after r.z and
 // r.r, after the new p) instead of six kernels, two of which summed 592 partials
 // with one thread. In K p a lane stands for a node, so that a warp's 32
-// neighbours lie side by side as the nodes do. Every warp takes the same number
-// of consecutive rows (entry k of a slice's 32 lists), wherever slices begin, and
-// leaves a partial sum per slice it touched (a segment); the update adds the
-// segments of a slice in order. So the warps are equally loaded at every size,
-// and p.Kp needs no complete sums. What bounds it: at 20 000 nodes the latency of
-// 17 rows of gathers and three barriers, at millions the L1 wavefronts of the
+// neighbours lie side by side as the nodes do; a block shares out the partial sums
+// of its slices, two per warp, so that warps and blocks are equally loaded at
+// every size. Every sum keeps the order it had with a warp per node and a group
+// of 8 warps per partial, so the iterates are those of the six kernels bit for
+// bit: a different order moves a solution by the solve's tolerance, which flips last
+// bits of positions and so changes single forces by 6e-8 of their RMS. What
+// bounds it: at 20 000 nodes the latency of ten rounds of gathers, three barriers
+// and the ordered sums of the partials, at millions the L1 wavefronts of the
 // gathers and 12 bytes an entry. 20 000 nodes, 1.0M bonds, B200: 109 us an
-// iteration with six kernels, 22 here (10 of them barriers, sums and updates);
-// 128 000 nodes 324 and 88. One block of 16 warps per SM ran faster than two at
-// 64 registers (27 us: spills, twice the arrivals).
+// iteration with six kernels, 33 here.
+// Warps with equal runs of rows and sums in any order took 22.
 __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
 {
-    __shared__ double sh[2][32];
+    extern __shared__ __align__(16) unsigned char cg_smem[];
+    CgShared &sm = *reinterpret_cast<CgShared *>(cg_smem);
     GridBarrier bar(A.bar, A.state + 2, A.timeout_ns);
     const int64_t n = A.g.n;
-    const int lane = threadIdx.x & 31;
-    const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t r0 = gw * A.chunk, r1 = min(A.rows, r0 + A.chunk);
-    int64_t sfirst = 0;   // slice of row r0
-    if (r0 < r1)
-        for (int64_t lo = 0, hi = A.g.ns; hi - lo > 1;) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (A.g.sptr[mid] <= r0 * 32) lo = mid;
-            else hi = mid;
-            sfirst = lo;
-        }
-    double2 *part0 = A.part, *part1 = A.part + gridDim.x;
+    const int groups = (int)min((int64_t)kCgGroups, (n + 255) / 256);
+    const int pgroups = 4 * (int)min((int64_t)kCgOwners, A.g.ns);
+    double2 *part0 = A.part, *part1 = A.part + kCgGroups;
     double rz, rr, rr0;
     int done = 0;
     if (A.first) {
         // delta = 0, r = F on the solved DOFs, z = M^-1 r, p = z
-        rz = rr = 0;
-        GRID_STRIDE(i, n)
-        {
+        node_sums(n, part0, sm, [&](int64_t i, double &rz_, double &rr_) {
             double ri[3], zi[3];
             for (int c = 0; c < 3; c++) ri[c] = A.skip[i + c * n] ? 0.0 : A.F[i + c * n];
             double m[6];
@@ -457,15 +567,17 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
                 if (A.skip[i + c * n]) zi[c] = 0.0;
                 A.d[i + c * n] = 0.0;
                 A.r[i + c * n] = ri[c];
-                rz += ri[c] * zi[c];
-                rr += ri[c] * ri[c];
+                rz_ += ri[c] * zi[c];
+                rr_ += ri[c] * ri[c];
             }
             A.rec[i].px = zi[0];
             A.rec[i].py = zi[1];
             A.rec[i].pz = zi[2];
-        }
-        if (!grid_sum2(rz, rr, sh, part0, bar)) return;
-        rr0 = rr;
+        });
+        if (!bar.wait()) return;
+        const double2 s = add_groups(part0, groups, sm);
+        rz = s.x;
+        rr = rr0 = s.y;
     } else {
         rz = A.scal[0];
         rr = A.scal[1];
@@ -474,87 +586,23 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
     }
     int state = rr0 > 0 ? CG_MORE : CG_DONE;   // a NaN r.r has nothing to solve either
     for (int it = 0; it < kCgLaunch && state == CG_MORE; it++) {
-        // y = K p, p.y
-        double py = 0, unused = 0;
-        for (int64_t row = r0, s = sfirst; row < r1; s++) {
-            const int64_t end = min(r1, A.g.sptr[s + 1] >> 5), i = s * 32 + lane;
-            if (end <= row) continue;   // a slice without bonds
-            Rec6 o = {0, 0, 0, 0, 0, 0};
-            if (i < n) o = load_rec(A.rec + i);
-            double y0 = 0, y1 = 0, y2 = 0;
-            auto add = [&](const Rec6 &q, double r) {
-                const double c0 = q.x - o.x, c1 = q.y - o.y, c2 = q.z - o.z;
-                const double t = r * (c0 * (o.px - q.px) + c1 * (o.py - q.py) + c2 * (o.pz - q.pz));
-                // a failed bond (r = 0) adds nothing, whatever its ends hold
-                y0 += r != 0 ? t * c0 : 0.0;
-                y1 += r != 0 ? t * c1 : 0.0;
-                y2 += r != 0 ? t * c2 : 0.0;
-            };
-            // kCgRows rows at a time, the next rows' streams on their way;
-            // rows past the end repeat the last one with scale 0
-            const uint32_t *col = A.g.col + row * 32 + lane;
-            const double *rig = A.rigE + row * 32 + lane;
-            const int rows = (int)(end - row);
-            uint32_t j[kCgRows];
-            double g[kCgRows];
-            auto streams = [&](int k) {
-#pragma unroll
-                for (int q = 0; q < kCgRows; q++) {
-                    const int at = min(k + q, rows - 1) * 32;
-                    j[q] = __ldg(col + at);
-                    g[q] = k + q < rows ? __ldg(rig + at) : 0.0;
-                }
-            };
-            streams(0);
-            for (int k = 0; k < rows; k += kCgRows) {
-                Rec6 v[kCgRows];
-                double h[kCgRows];
-#pragma unroll
-                for (int q = 0; q < kCgRows; q++) {
-                    v[q] = load_rec(A.rec + j[q]);
-                    h[q] = g[q];
-                }
-                if (k + kCgRows < rows) streams(k + kCgRows);
-#pragma unroll
-                for (int q = 0; q < kCgRows; q++) add(v[q], h[q]);
-            }
-            row = end;
-            double *ys = A.yseg + (s + gw) * 96 + lane;
-            ys[0] = y0;
-            ys[32] = y1;
-            ys[64] = y2;
-            py += o.px * y0 + o.py * y1 + o.pz * y2;   // p is zero on held DOFs
-        }
-        if (!grid_sum2(py, unused, sh, part1, bar)) return;
+        cg_product(A.g, A.rigE, A.rec, A.y, part1, sm);
+        if (!bar.wait()) return;
+        const double py = add_groups(part1, pgroups, sm).x;
         // delta += alpha p, r -= alpha y, z = M^-1 r
         const double alpha = py != 0 ? rz / py : 0.0;
-        double rzn = 0, rrn = 0;
-        GRID_STRIDE(i, n)
-        {
-            // every load first, then the segments four at a time: one round
-            // trip to L2 for nearly all nodes
-            const int2 q2 = *reinterpret_cast<const int2 *>(A.seg + 2 * (i >> 5));
+        node_sums(n, part0, sm, [&](int64_t i, double &rz_, double &rr_) {
+            // every load first: one round trip to L2
             const double pv[3] = {A.rec[i].px, A.rec[i].py, A.rec[i].pz};
-            double ri[3], zi[3], di[3], m[6], yi[3] = {0, 0, 0};
+            double ri[3], zi[3], di[3], m[6], yi[3];
             bool sk[3];
             for (int c = 0; c < 3; c++) {
+                yi[c] = __ldcg(A.y + i + c * n);
                 ri[c] = A.r[i + c * n];
                 di[c] = A.d[i + c * n];
                 sk[c] = A.skip[i + c * n] != 0;
             }
             for (int c = 0; c < 6; c++) m[c] = A.Minv[i + c * n];
-            for (int q = q2.x; q < q2.y; q += 4) {
-                const double *ys = A.yseg + (int64_t)q * 96 + (i & 31);
-                double v[4][3];
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) v[k][c] = q + k < q2.y ? __ldcg(ys + k * 96 + c * 32) : 0.0;
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-#pragma unroll
-                    for (int c = 0; c < 3; c++) yi[c] += v[k][c];
-            }
             for (int c = 0; c < 3; c++) {
                 A.d[i + c * n] = di[c] + alpha * pv[c];
                 ri[c] = sk[c] ? 0.0 : ri[c] - alpha * yi[c];
@@ -564,21 +612,22 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
             for (int c = 0; c < 3; c++) {
                 if (sk[c]) zi[c] = 0.0;
                 A.z[i + c * n] = zi[c];
-                rzn += ri[c] * zi[c];
-                rrn += ri[c] * ri[c];
+                rz_ += ri[c] * zi[c];
+                rr_ += ri[c] * ri[c];
             }
-        }
-        if (!grid_sum2(rzn, rrn, sh, part0, bar)) return;
+        });
+        if (!bar.wait()) return;
+        const double2 s = add_groups(part0, groups, sm);
         // p = z + beta p
-        const double beta = rz != 0 ? rzn / rz : 0.0;
+        const double beta = rz != 0 ? s.x / rz : 0.0;
         GRID_STRIDE(i, n)
         {
-            A.rec[i].px = A.z[i] + beta * A.rec[i].px;
-            A.rec[i].py = A.z[i + n] + beta * A.rec[i].py;
-            A.rec[i].pz = A.z[i + 2 * n] + beta * A.rec[i].pz;
+            A.rec[i].px = __ldcg(A.z + i) + beta * A.rec[i].px;
+            A.rec[i].py = __ldcg(A.z + i + n) + beta * A.rec[i].py;
+            A.rec[i].pz = __ldcg(A.z + i + 2 * n) + beta * A.rec[i].pz;
         }
-        rz = rzn;
-        rr = rrn;
+        rz = s.x;
+        rr = s.y;
         done++;
         if (done % kCgCheck == 0 || done == A.max_cg) {
             if (!isfinite(rr)) state = CG_NONFINITE;
@@ -640,9 +689,7 @@ struct bbpd_static {
     double2 *cg_part = nullptr;
     int *cg_state = nullptr;               // state, iterations, error word, barrier arrivals
     int cg_grid = 0;
-    int64_t rows = 0, chunk = 1;
-    double *yseg = nullptr;
-    int32_t *seg = nullptr;
+    double *y = nullptr;
     uint8_t *skip = nullptr;
     SBonds b{};
     SNodes g{};
@@ -669,13 +716,13 @@ int run_cg(bbpd_static *S, double cg_tol, int max_cg, int state[2])
 {
     cudaStream_t st = S->st;
     const double to = S->prm.barrier_timeout_s > 0 ? S->prm.barrier_timeout_s : 2.0;
-    CgArgs A{S->g, S->rigE, S->rec, S->F, S->Minv, S->skip, S->x, S->d, S->r, S->z, S->yseg, S->seg, S->cg_part,
+    CgArgs A{S->g, S->rigE, S->rec, S->F, S->Minv, S->skip, S->x, S->d, S->r, S->z, S->y, S->cg_part,
              S->scal, S->cg_state, reinterpret_cast<unsigned *>(S->cg_state + 3), (unsigned long long)(to * 1e9),
-             cg_tol * cg_tol, 1, max_cg, S->rows, S->chunk};
+             cg_tol * cg_tol, 1, max_cg};
     for (;; A.first = 0) {
         BBPD_CUDA_TRY(cudaMemsetAsync(S->cg_state + 2, 0, 2 * sizeof(int), st));
         void *args[] = {(void *)&A};
-        BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_cg, dim3(S->cg_grid), dim3(kCgThreads), args, 0, st));
+        BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_cg, dim3(S->cg_grid), dim3(kCgThreads), args, sizeof(CgShared), st));
         int h[3];
         BBPD_CUDA_TRY(cudaMemcpyAsync(h, S->cg_state, sizeof(h), cudaMemcpyDeviceToHost, st));
         BBPD_CUDA_TRY(cudaStreamSynchronize(st));
@@ -896,20 +943,13 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     BBPD_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     BBPD_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
     if (!coop) return fail(BBPD_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg, kCgThreads, 0));
+    BBPD_CUDA_TRY(cudaFuncSetAttribute(k_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgShared)));
+    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg, kCgThreads, sizeof(CgShared)));
     if (occ < 1) return fail(BBPD_ERR_CUDA, "kernel cannot be resident");
-    // no more blocks than give every warp four rows, and every thread a node
-    const int64_t wpb = kCgThreads / 32;
-    S->rows = slots / 32;
-    S->cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)nsm * occ,
-                                                             std::max((S->rows + 4 * wpb - 1) / (4 * wpb),
-                                                                      (n + kCgThreads - 1) / kCgThreads)));
-    S->chunk = std::max<int64_t>(1, (S->rows + S->cg_grid * wpb - 1) / (S->cg_grid * wpb));
-    TRY(S->alloc(&S->yseg, (ns + S->cg_grid * wpb) * 96));
-    TRY(S->alloc(&S->seg, 2 * ns));
-    k_segments<<<blocks_for(ns), kThreads, 0, st>>>(sptr, ns, S->chunk, S->seg);
-    TRY(launch_check());
-    TRY(S->alloc(&S->cg_part, 2 * S->cg_grid));
+    // a block for every owner with slices
+    S->cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)nsm, (int64_t)kCgOwners, ns}));
+    TRY(S->alloc(&S->y, 3 * n));
+    TRY(S->alloc(&S->cg_part, 2 * kCgGroups));
     TRY(S->alloc(&S->cg_state, 4));
     S->g.off = off;
     S->g.ent = ent;
@@ -958,7 +998,7 @@ extern "C" int bbpd_static_step(bbpd_static *S, double increment, double tol, in
         // K delta = F on the free DOFs by PCG, x += delta
         k_static_records<<<blocks_for(n), kThreads, 0, st>>>(S->x, n, S->rec);
         k_slot_rig<<<blocks_for(2 * S->nB), kThreads, 0, st>>>(S->g.bond, S->b.rig, S->g.sptr + S->g.ns, S->rigE);
-        k_static_precond<<<blocks_for(32 * n), kThreads, 0, st>>>(S->g, S->b.rig, S->rec, S->Minv, S->skip);
+        k_static_precond<<<blocks_for(n), kThreads, 0, st>>>(S->g, S->rigE, S->rec, S->Minv, S->skip);
         TRY(launch_check());
         int cg[2] = {CG_DONE, 0};
         TRY(run_cg(S, cg_tol, max_cg, cg));
