@@ -116,13 +116,16 @@ __global__ void k_cell_of(const double *__restrict__ X, int64_t n, Grid g, uint3
     }
 }
 
-// start[c]: first sorted position whose cell is c or later, for c in [0, ncell]
-__global__ void k_cell_starts(const uint32_t *__restrict__ scell, int64_t n, int64_t ncell, uint32_t *start)
+// Cell c holds the sorted positions [first, end): .x = first, .y = ~end, both
+// all ones where the cell is empty (so the caller fills the table with ones, and a
+// cloud with few points in many cells costs no walk over them)
+__global__ void k_cell_bounds(const uint32_t *__restrict__ scell, int64_t n, uint2 *cells)
 {
-    GRID_STRIDE(q, n + 1)
+    GRID_STRIDE(q, n)
     {
-        const int64_t c0 = q == 0 ? 0 : (int64_t)scell[q - 1] + 1, c1 = q == n ? ncell : (int64_t)scell[q];
-        for (int64_t c = c0; c <= c1; c++) start[c] = (uint32_t)q;
+        const uint32_t c = scell[q];
+        if (q == 0 || scell[q - 1] != c) cells[c].x = (uint32_t)q;
+        if (q == n - 1 || scell[q + 1] != c) cells[c].y = ~(uint32_t)(q + 1);
     }
 }
 
@@ -142,7 +145,8 @@ struct Cloud {
     int64_t n;
     double horizon;
     Grid g;
-    const uint32_t *scell, *snode, *start;
+    const uint32_t *scell, *snode;
+    const uint2 *cells;
     const double *sx;   // positions in sorted order, x then y then z
 };
 
@@ -159,7 +163,8 @@ __device__ __forceinline__ void scan_family(const Cloud &C, int64_t q, int lane,
     for (int64_t z = cz > 0 ? cz - 1 : 0; z <= cz + 1 && z < nz; z++)
         for (int64_t y = cy > 0 ? cy - 1 : 0; y <= cy + 1 && y < ny; y++) {
             const int64_t row = nx * (y + ny * z);
-            const uint32_t a = C.start[row + xa], b = C.start[row + xb + 1];
+            const uint2 u = C.cells[row + xa], v = C.cells[row + cx], w = C.cells[row + xb];
+            const uint32_t a = min(min(u.x, v.x), w.x), b = ~min(min(u.y, v.y), w.y);
             for (uint32_t r0 = a; r0 < b; r0 += 32) {
                 const uint32_t r = r0 + lane;
                 int64_t j = i;
@@ -561,7 +566,8 @@ struct Horizons {
             g.h *= 1.25;
         }
         const int64_t ncell = g.nc[0] * g.nc[1] * g.nc[2];
-        uint32_t *cell = nullptr, *node = nullptr, *scell = nullptr, *snode = nullptr, *start = nullptr;
+        uint32_t *cell = nullptr, *node = nullptr, *scell = nullptr, *snode = nullptr;
+        uint2 *cells = nullptr;
         double *sx = nullptr;
         int *dlargest = nullptr;
         TRY(s.get(&cell, n));
@@ -575,16 +581,17 @@ struct Horizons {
         uint8_t *tmp = nullptr;
         TRY(s.get(&tmp, tb));
         BBPD_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tb, cell, scell, node, snode, n, 0, bits_for(ncell), st));
-        TRY(s.get(&start, ncell + 1));
+        TRY(s.get(&cells, ncell));
+        BBPD_CUDA_TRY(cudaMemsetAsync(cells, 0xFF, sizeof(uint2) * ncell, st));
         TRY(s.get(&sx, 3 * n));
-        k_cell_starts<<<blocks_for(n + 1), kThreads, 0, st>>>(scell, n, ncell, start);
+        k_cell_bounds<<<blocks_for(n), kThreads, 0, st>>>(scell, n, cells);
         k_sorted_positions<<<blocks_for(n), kThreads, 0, st>>>(X, n, snode, sx);
         TRY(launch_check());
         TRY(s.get(&fam, n));
         TRY(s.get(&fwd, n));
         TRY(s.get(&dlargest, 1));
         BBPD_CUDA_TRY(cudaMemsetAsync(dlargest, 0, sizeof(int), st));
-        C = Cloud{n, r, g, scell, snode, start, sx};
+        C = Cloud{n, r, g, scell, snode, cells, sx};
         k_horizon_count<<<blocks_for(32 * n), kThreads, 0, st>>>(C, fam, fwd, dlargest);
         TRY(launch_check());
         int64_t *w = nullptr;

@@ -38,6 +38,8 @@
 //            folded by the warp that completes them, the root giving the
 //            damping coefficient cn; barrier; phase B applies the central-
 //            difference half-step update; barrier.
+// A beam of few slices runs split_kernel instead: a block of warps shares each
+// slice (its comment has the details); layout, arithmetic and order are the same.
 // Grid barriers spin with a time limit; on expiry they set an error flag and
 // the kernel returns early (status BBPD_ERR_TIMEOUT), never hanging.
 #include "bbpd_internal.h"
@@ -485,15 +487,10 @@ __device__ __forceinline__ void law_update(const Dev &d, int64_t e, int bt, uint
 // when it changes, bond force with the NaN guards of calculatebondforcesMex.c.
 // Bonds whose kinematics the branch-free pass cannot give come here, and in the
 // FP32 form those that need the law.
-#ifdef BBPD_GENERAL_OUTLINE
-#define BBPD_GENERAL_ATTR __noinline__
-#else
-#define BBPD_GENERAL_ATTR __forceinline__
-#endif
 template <int LAW, int PREC>
-__device__ BBPD_GENERAL_ATTR double3 entry_general(const Dev &d, int64_t e, uint32_t w, uint32_t sv,
-                                              DictEntry g, double scb, double xi, double yi,
-                                              double zi, double xj, double yj, double zj)
+__device__ __forceinline__ double3 entry_general(const Dev &d, int64_t e, uint32_t w, uint32_t sv,
+                                                 DictEntry g, double scb, double xi, double yi,
+                                                 double zi, double xj, double yj, double zj)
 {
     const LawScalars &P = d.P;
     const int bt = (w >> BT_SHIFT) & 3;

@@ -51,6 +51,23 @@ def test_horizons_vs_oracle_point_clouds(cloud):
     assert got[3].shape[0] > 1000
 
 
+@pytest.mark.parametrize("members", [1, 3, 31, 32, 33, 127, 129, 254, 255, 256, 257, 300])
+def test_horizons_family_sizes_and_empty_cells(members):
+    """Families around a warp's 32 candidates, a rank pass's 128 members and the
+    256 a warp ranks at most (more are sorted): two clusters whose points all see
+    one another, far apart in a grid of 7M cells, nearly all empty."""
+    rng = np.random.default_rng(members)
+    a = rng.uniform(-0.1, 0.1, (members + 1, 3))
+    b = rng.uniform(-0.1, 0.1, (members // 2 + 1, 3)) + [300.0, 230.0, 100.0]
+    X = rng.permutation(np.concatenate([a, b]))
+    got = G.buildhorizons(X, 1.0)
+    want = oracle_horizons(X, 1.0)
+    for name, p, q in zip(("nFAMILYMEMBERS", "NODEFAMILYPOINTERS", "NODEFAMILY", "BONDLIST", "UNDEFORMEDLENGTH"),
+                          got, want):
+        assert same(p, q), name
+    assert int(np.max(got[0])) == members
+
+
 def test_horizons_match_lattice_builder():
     """20 000 nodes, 1.0M bonds (the 100 x 10 x 20 beam): bit-identical with the
     lattice builder; the arrays cross the host boundary in staged chunks."""
