@@ -136,7 +136,7 @@ def test_static_other_laws_vs_oracle(law, steps):
 # 70 nodes have lost their bonds (slices without a row)
 @pytest.mark.parametrize("nx,ny,nz,cut", [(6, 2, 2, 0), (13, 3, 5, 0), (40, 6, 8, 0), (30, 4, 6, 70)])
 def test_static_solve_sizes_vs_oracle(nx, ny, nz, cut):
-    """The linear solve where its rows, slices and segments meet differently."""
+    """The linear solve where its rows and slices meet differently."""
     inp = dict(bb.beam.build(bb.beam.small(nx=nx, ny=ny, nz=nz)))
     if cut:   # the top layer's end, away from the loaded nodes
         keep = (inp["BONDLIST"] <= inp["nNodes"] - cut).all(axis=1)
@@ -156,4 +156,37 @@ def test_static_solve_sizes_vs_oracle(nx, ny, nz, cut):
         assert sg.converged and so["converged"], (step, sg.residual, sg.reaction)
         ug, uo = g.get("displacement"), o.get("displacement")
         assert np.abs(ug - uo).max() <= 1e-8 * np.abs(uo).max(), step
+    g.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz,copies", [(20, 4, 6, 2), (12, 4, 4, 3)])
+def test_static_solve_long_lists_vs_oracle(nx, ny, nz, copies):
+    """Lists of more than 128 entries: every bond several times, its stiffness
+    shared out."""
+    inp = dict(bb.beam.build(bb.beam.small(nx=nx, ny=ny, nz=nz)))
+    inp["BONDSTIFFNESS"] = inp["BONDSTIFFNESS"] / copies
+    for k in ("UNDEFORMEDLENGTH", "BONDSTIFFNESS", "VOLUMECORRECTIONFACTORS"):
+        inp[k] = np.tile(inp[k], copies)
+    inp["BONDLIST"] = np.asfortranarray(np.tile(inp["BONDLIST"], (copies, 1)))
+    inp["nBonds"] *= copies
+    g = StaticSolver(inp, law="linear", sc=1.0)
+    o = StaticOracle(inp, law="linear", sc=1.0)
+    sg = g.step(-1e-6, tol=1e-9, **CG)
+    so = o.step(-1e-6, tol=1e-9)
+    assert sg.converged and so["converged"], (sg.residual, sg.reaction)
+    ug, uo = g.get("displacement"), o.get("displacement")
+    assert np.abs(ug - uo).max() <= 1e-8 * np.abs(uo).max()
+    g.close()
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(50, 8, 12), (100, 12, 22)])
+def test_static_solve_many_slices(nx, ny, nz):
+    """More slices than the 148 that have a block of their own, and more than a
+    block multiplies at a time: the nodal forces, summed by another kernel, are in
+    equilibrium to 1e-6 of the reaction, which only a solved system gives (the
+    rounding of the positions alone leaves about 1e-9)."""
+    inp = bb.beam.build(bb.beam.small(nx=nx, ny=ny, nz=nz))
+    g = StaticSolver(inp, law="linear", sc=1.0)
+    st = g.step(-1e-6, tol=1e-6, **CG)
+    assert st.converged and st.newton_iterations >= 1 and st.residual <= 1e-6 * st.reaction
     g.close()
