@@ -305,8 +305,9 @@ __global__ void k_damageenergy(const double *__restrict__ BS, const double *__re
 
 // ---- nodal force plan ----
 
+template <class ENT>
 __global__ void k_plan_keys(const double *__restrict__ bl, int64_t nB, int64_t nN,
-                            int32_t *keys, int64_t *vals, int *bad)
+                            int32_t *keys, ENT *vals, int *bad)
 {
     GRID_STRIDE(k, nB)
     {
@@ -332,16 +333,16 @@ __global__ void k_plan_count(const int32_t *keys, int64_t n, int32_t *cnt)
 // bit set where bond k belongs to another OpenMP chunk than the entry before
 // it in its node's list (calculatenodalforcesopenmpMex.c:39 static schedule)
 template <class ENT>
-__global__ void k_plan_pack(const int64_t *__restrict__ sorted, const int32_t *__restrict__ node, int64_t n, int64_t nB,
+__global__ void k_plan_pack(const ENT *__restrict__ sorted, const int32_t *__restrict__ node, int64_t n, int64_t nB,
                             int T, ENT *ent)
 {
     constexpr ENT kFlag = (ENT)1 << (8 * sizeof(ENT) - 1);
     GRID_STRIDE(p, n)
     {
-        const int64_t v = sorted[p];
+        const ENT v = sorted[p];
         const bool first = p == 0 || node[p - 1] != node[p];
-        const bool flag = !first && omp_chunk_of(v >> 1, nB, T) != omp_chunk_of(sorted[p - 1] >> 1, nB, T);
-        ent[p] = (ENT)v | (flag ? kFlag : (ENT)0);
+        const bool flag = !first && omp_chunk_of((int64_t)(v >> 1), nB, T) != omp_chunk_of((int64_t)(sorted[p - 1] >> 1), nB, T);
+        ent[p] = v | (flag ? kFlag : (ENT)0);
     }
 }
 
@@ -572,10 +573,10 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
     p->nB = nB; p->nN = nN; p->T = nChunks;
     int64_t ne = 2 * nB;
     int32_t *keys = nullptr, *keys2 = nullptr, *cnt = nullptr;
-    int64_t *vals = nullptr, *vals2 = nullptr;
+    void *vals = nullptr, *vals2 = nullptr;
     int *bad = nullptr;
     void *tmp = nullptr;
-    size_t tmpb = 0, tmpb2 = 0;
+    size_t tmpb = 0;
     const bool narrow = ne < (int64_t)1 << 31;   // the top bit is the chunk flag
     cudaError_t e = cudaSuccess;
 #define PLAN_TRY(x) do { e = (x); if (e != cudaSuccess) goto fail_; } while (0)
@@ -589,19 +590,23 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
     if (ne > 0) {
         PLAN_TRY(cudaMalloc(&keys, sizeof(int32_t) * (size_t)ne));
         PLAN_TRY(cudaMalloc(&keys2, sizeof(int32_t) * (size_t)ne));
-        PLAN_TRY(cudaMalloc(&vals, sizeof(int64_t) * (size_t)ne));
-        PLAN_TRY(cudaMalloc(&vals2, sizeof(int64_t) * (size_t)ne));
-        k_plan_keys<<<blocks_for(nB), kThreads, 0, st>>>(bl, nB, nN, keys, vals, bad);
-        // stable radix sort by node keeps each node's entries in bond order
-        PLAN_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmpb, keys, keys2, vals, vals2, ne, 0, 32, st));
-        PLAN_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmpb2, cnt, cnt, nN + 1, st));
-        if (tmpb2 > tmpb) tmpb = tmpb2;
-        PLAN_TRY(cudaMalloc(&tmp, tmpb));
-        PLAN_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmpb, keys, keys2, vals, vals2, ne, 0, 32, st));
-        k_plan_count<<<blocks_for(ne), kThreads, 0, st>>>(keys, ne, cnt);
-        if (narrow) k_plan_pack<<<blocks_for(ne), kThreads, 0, st>>>(vals2, keys2, ne, nB, nChunks, p->ent32);
-        else k_plan_pack<<<blocks_for(ne), kThreads, 0, st>>>(vals2, keys2, ne, nB, nChunks, p->ent64);
-        PLAN_TRY(cudaGetLastError());
+        auto entries = [&](auto *ent) {   // ent: the plan's entries, 32 or 64 bits each
+            using ENT = std::remove_pointer_t<decltype(ent)>;
+            cudaError_t r = cudaMalloc(&vals, sizeof(ENT) * (size_t)ne);
+            if (r == cudaSuccess) r = cudaMalloc(&vals2, sizeof(ENT) * (size_t)ne);
+            if (r != cudaSuccess) return r;
+            ENT *v = (ENT *)vals, *v2 = (ENT *)vals2;
+            k_plan_keys<<<blocks_for(nB), kThreads, 0, st>>>(bl, nB, nN, keys, v, bad);
+            // stable radix sort by node keeps each node's entries in bond order
+            r = cub::DeviceRadixSort::SortPairs(nullptr, tmpb, keys, keys2, v, v2, ne, 0, 32, st);
+            if (r == cudaSuccess) r = cudaMalloc(&tmp, tmpb);
+            if (r == cudaSuccess) r = cub::DeviceRadixSort::SortPairs(tmp, tmpb, keys, keys2, v, v2, ne, 0, 32, st);
+            if (r != cudaSuccess) return r;
+            k_plan_count<<<blocks_for(ne), kThreads, 0, st>>>(keys, ne, cnt);
+            k_plan_pack<<<blocks_for(ne), kThreads, 0, st>>>(v2, keys2, ne, nB, nChunks, ent);
+            return cudaGetLastError();
+        };
+        PLAN_TRY(narrow ? entries(p->ent32) : entries(p->ent64));
     }
     {
         // row pointers: exclusive scan of the counts (64-bit)
