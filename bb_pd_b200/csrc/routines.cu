@@ -1,7 +1,8 @@
 // Per-routine CUDA kernels: one entry point per reference MEX routine (and per
 // MATLAB-only routine of the hot path), with the reference's argument meaning
 // and in-place semantics. Bond routines run one thread per bond, node routines
-// one thread per node. The nodal force sum is node-centric (nodalsum.cuh): a plan
+// one thread per node. The nodal force sum is node-centric (nodalsum.cuh, or a
+// thread per node where the lists are short): a plan
 // holds each node's bonds in bond order and the node adds them in the reference's
 // OpenMP order, so no atomics are needed and the result is bit-identical.
 //
@@ -347,7 +348,34 @@ __global__ void k_plan_pack(const ENT *__restrict__ sorted, const int32_t *__res
 }
 
 // nodalForce[n] += thread partials in thread order
-// (calculatenodalforcesopenmpMex.c:56-80). 7.1M bonds, 128 000 nodes on B200:
+// (calculatenodalforcesopenmpMex.c:56-80): a thread per node, for short lists.
+template <class ENT>
+__global__ void __launch_bounds__(kThreads) k_nodalforces_short(const int64_t *__restrict__ rp, const ENT *__restrict__ ent,
+                                                                int64_t nN, double *F, const double *__restrict__ fX,
+                                                                const double *__restrict__ fY, const double *__restrict__ fZ)
+{
+    constexpr ENT kFlag = (ENT)1 << (8 * sizeof(ENT) - 1);
+    GRID_STRIDE(n, nN)
+    {
+        const int64_t p0 = rp[n], p1 = rp[n + 1];
+        if (p0 == p1) continue;
+        double tx = F[n], ty = F[n + nN], tz = F[n + 2 * nN];
+        double ax = 0.0, ay = 0.0, az = 0.0;
+        for (int64_t p = p0; p < p1; p++) {
+            const ENT v = ent[p];
+            const int64_t k = (int64_t)((v & ~kFlag) >> 1);
+            if (v & kFlag) {   // partial of the previous OpenMP thread is complete
+                tx = tx + ax; ty = ty + ay; tz = tz + az;
+                ax = ay = az = 0.0;
+            }
+            if (v & 1) { ax = ax - fX[k]; ay = ay - fY[k]; az = az - fZ[k]; }
+            else       { ax = ax + fX[k]; ay = ay + fY[k]; az = az + fZ[k]; }
+        }
+        F[n] = tx + ax; F[n + nN] = ty + ay; F[n + 2 * nN] = tz + az;
+    }
+}
+
+// The same by warps (nodalsum.cuh). 7.1M bonds, 128 000 nodes on B200:
 // 265 us with a thread per node, 109 now; 50 000 bonds, 1 953 nodes: 117 us, 10 now
 // (under ncu, caches cold).
 template <class ENT>
@@ -402,7 +430,21 @@ struct bbpd_nodal_plan {
     int64_t *rp = nullptr;     // nN + 1
     uint32_t *ent32 = nullptr; // 2 nB entries, 32-bit where they fit
     uint64_t *ent64 = nullptr;
+    bool brief = false;        // k_nodalforces_short: see short_lists
 };
+
+// Where a thread per node adds faster than a warp for four: the warp's round of 32
+// entries a node is mostly padding on lists of a few, so from 65 536 nodes on
+// (enough threads to fill the GPU) and up to 20 entries a node the thread wins. One
+// list must not hold its thread much longer than the rest, hence at most 64. us on B200, warp
+// against thread: 1M nodes of 6 entries (a lattice's nearest neighbours) 201 / 40,
+// of 18 232 / 138, of 26 234 / 249, of 31 288 / 466; 200 000 nodes of 6 41 / 13, of
+// 25 60 / 58, of 31 72 / 94; 20 000 nodes of 6 12.9 / 10.3, of 17 13.2 / 13.6, of 12
+// to random neighbours 14.8 / 18.2; 2 000 nodes of 22 14.8 / 15.6.
+static bool short_lists(int64_t nN, int64_t entries, int64_t longest)
+{
+    return nN >= 65536 && entries <= 20 * nN && longest <= 64;
+}
 
 // ---- device-pointer entry points ----
 
@@ -621,9 +663,14 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
             return fail(BBPD_ERR_ARG, "BONDLIST holds a node id that is not an integer in [1, nNodes] or a self-bond");
         }
         std::vector<int64_t> hr((size_t)nN + 1);
-        int64_t acc = 0;
-        for (int64_t i = 0; i < nN; i++) { hr[i] = acc; acc += hc[i]; }
+        int64_t acc = 0, longest = 0;
+        for (int64_t i = 0; i < nN; i++) {
+            hr[i] = acc;
+            acc += hc[i];
+            longest = std::max<int64_t>(longest, hc[i]);
+        }
         hr[nN] = acc;
+        p->brief = short_lists(nN, ne, longest);
         PLAN_TRY(cudaMemcpyAsync(p->rp, hr.data(), sizeof(int64_t) * (size_t)(nN + 1), cudaMemcpyHostToDevice, st));
         PLAN_TRY(cudaStreamSynchronize(st));
     }
@@ -653,9 +700,13 @@ extern "C" int bbpd_dev_calculatenodalforces(const bbpd_nodal_plan *p, double *F
 {
     if (!p) return fail(BBPD_ERR_ARG, "null plan");
     if (p->nN == 0) return BBPD_OK;
-    const int blocks = blocks_for((p->nN + kNodes - 1) / kNodes * 32);
-    if (p->ent64) k_nodalforces<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, p->ent64, p->nN, F, fX, fY, fZ);
-    else k_nodalforces<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, p->ent32, p->nN, F, fX, fY, fZ);
+    const int blocks = blocks_for(p->brief ? p->nN : (p->nN + kNodes - 1) / kNodes * 32);
+    auto sum = [&](const auto *ent) {
+        if (p->brief) k_nodalforces_short<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, ent, p->nN, F, fX, fY, fZ);
+        else k_nodalforces<<<blocks, kThreads, 0, as_stream(stream)>>>(p->rp, ent, p->nN, F, fX, fY, fZ);
+    };
+    if (p->ent64) sum(p->ent64);
+    else sum(p->ent32);
     return launch_check();
 }
 

@@ -117,6 +117,31 @@ def test_nodalforces_list_lengths(nN, hubs, T):
     assert same(F, Fo)
 
 
+@pytest.mark.parametrize("nN,ring,hub", [(65535, 1, 0), (65536, 1, 0), (65536, 10, 0), (65536, 11, 0), (65537, 9, 46),
+                                         (65537, 9, 47)])
+@pytest.mark.parametrize("T", [1, 8])
+def test_nodalforces_short_lists(nN, ring, hub, T):
+    """Both sides of the lines between a thread and a warp per list: 65 536 nodes,
+    20 entries a node, 64 entries in the longest list. Every node has `ring` bonds
+    to each neighbour of a ring, and node 5 `hub` more; shuffled bond order."""
+    rng = np.random.default_rng(ring + hub)
+    i = np.tile(np.arange(nN), ring)
+    rows = np.stack([i, (i + 1) % nN], 1)
+    if hub:
+        rows = np.concatenate([rows, np.stack([np.full(hub, 5), 100 + np.arange(hub)], 1)])
+    flip = rng.random(len(rows)) < 0.5
+    rows[flip] = rows[flip][:, ::-1]
+    bl = np.asfortranarray(rows[rng.permutation(len(rows))] + 1.0)
+    nB = len(bl)
+    f = [rng.normal(0, 1e3, nB) for _ in range(3)]
+    f[0][::3], f[1][::4] = 0.0, -0.0
+    F = np.asfortranarray(np.where(rng.random((nN, 3)) < 0.5, -0.0, rng.normal(0, 1, (nN, 3))))
+    Fo = F.copy(order="F")
+    (R.calculatenodalforcesopenmpMex if T == 8 else R.calculatenodalforcesMex)(bl, F, *f)
+    po.lib().orc_nodalforces_chunked(nB, nN, P(bl), P(Fo), P(f[0]), P(f[1]), P(f[2]), T)
+    assert same(F, Fo)
+
+
 def test_eulercromer_golden():
     g = gold("eulercromer")
     nN = g["F"].shape[0]
