@@ -51,6 +51,20 @@ def test_horizons_vs_oracle_point_clouds(cloud):
     assert got[3].shape[0] > 1000
 
 
+@pytest.mark.parametrize("per_cell", [0.2, 1.0, 1.2, 2.4, 3.6, 7.0])
+def test_horizons_sparse_clouds(per_cell):
+    """A few points per cell: the 27 cells around a point hold some 5 to 190
+    candidates, so 32 of them reach over several, empty and half-empty runs of cells."""
+    rng = np.random.default_rng(int(10 * per_cell))
+    r = 0.125
+    X = rng.uniform(0, 1, (int(512 * per_cell), 3))
+    got = G.buildhorizons(X, r)
+    want = oracle_horizons(X, r)
+    for name, a, b in zip(("nFAMILYMEMBERS", "NODEFAMILYPOINTERS", "NODEFAMILY", "BONDLIST", "UNDEFORMEDLENGTH"),
+                          got, want):
+        assert same(a, b), name
+
+
 @pytest.mark.parametrize("members", [1, 3, 31, 32, 33, 127, 129, 254, 255, 256, 257, 300])
 def test_horizons_family_sizes_and_empty_cells(members):
     """Families around a warp's 32 candidates, a rank pass's 128 members and the
