@@ -689,6 +689,7 @@ struct bbpd_static {
     double2 *cg_part = nullptr;
     int *cg_state = nullptr;               // state, iterations, error word, barrier arrivals
     int cg_grid = 0;
+    unsigned long long cg_limit_ns = 0;    // of a barrier wait
     double *y = nullptr;
     uint8_t *skip = nullptr;
     SBonds b{};
@@ -715,9 +716,8 @@ namespace {
 int run_cg(bbpd_static *S, double cg_tol, int max_cg, int state[2])
 {
     cudaStream_t st = S->st;
-    const double to = S->prm.barrier_timeout_s > 0 ? S->prm.barrier_timeout_s : 2.0;
     CgArgs A{S->g, S->rigE, S->rec, S->F, S->Minv, S->skip, S->x, S->d, S->r, S->z, S->y, S->cg_part,
-             S->scal, S->cg_state, reinterpret_cast<unsigned *>(S->cg_state + 3), (unsigned long long)(to * 1e9),
+             S->scal, S->cg_state, reinterpret_cast<unsigned *>(S->cg_state + 3), S->cg_limit_ns,
              cg_tol * cg_tol, 1, max_cg};
     for (;; A.first = 0) {
         BBPD_CUDA_TRY(cudaMemsetAsync(S->cg_state + 2, 0, 2 * sizeof(int), st));
@@ -948,6 +948,11 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     if (occ < 1) return fail(BBPD_ERR_CUDA, "kernel cannot be resident");
     // a block for every owner with slices
     S->cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)nsm, (int64_t)kCgOwners, ns}));
+    // A solve that makes progress never waits this long: 10 s, and 0.1 us for every
+    // row of 32 entries, should one block have them all (16 warps take one in 0.02 us).
+    // barrier_timeout_s, the limit of the time-stepping kernels, may be short; it
+    // has no say here.
+    S->cg_limit_ns = 10000000000ull + 100ull * (unsigned long long)(slots >> 5);
     TRY(S->alloc(&S->y, 3 * n));
     TRY(S->alloc(&S->cg_part, 2 * kCgGroups));
     TRY(S->alloc(&S->cg_state, 4));

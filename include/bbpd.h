@@ -353,7 +353,8 @@ typedef struct bbpd_params {
     double applied_final;     /* BBPD_AMP_SMOOTHSTEP: final displacement */
     int64_t n_time_steps;     /* BBPD_AMP_SMOOTHSTEP: final step */
     double guard_band;        /* BBPD_PREC_FP32: FP64 recheck when |s - sc| < guard_band */
-    double barrier_timeout_s; /* device grid-barrier wait limit (0 = 2 s) */
+    double barrier_timeout_s; /* device grid-barrier wait limit of the time
+                                 stepping (0 = 2 s); the static solver has its own */
 } bbpd_params;
 
 /* Fill params with the reference defaults (law exponential k=25 alpha=0.25,

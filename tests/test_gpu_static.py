@@ -190,3 +190,27 @@ def test_static_solve_many_slices(nx, ny, nz):
     st = g.step(-1e-6, tol=1e-6, **CG)
     assert st.converged and st.newton_iterations >= 1 and st.residual <= 1e-6 * st.reaction
     g.close()
+
+
+def with_hubs(inp, hubs):
+    """The input with a weak bond from each node of `hubs` to every other node."""
+    inp = dict(inp)
+    n, X = inp["nNodes"], inp["undeformedCoordinates"]
+    i = np.repeat(hubs, n - 1)
+    j = np.concatenate([np.delete(np.arange(n), h) for h in hubs])
+    inp["BONDLIST"] = np.asfortranarray(np.concatenate([inp["BONDLIST"], np.stack([i, j], 1) + 1.0]))
+    inp["UNDEFORMEDLENGTH"] = np.concatenate([inp["UNDEFORMEDLENGTH"], np.sqrt(((X[i] - X[j]) ** 2).sum(1))])
+    inp["BONDSTIFFNESS"] = np.concatenate([inp["BONDSTIFFNESS"], np.full(i.size, 1e-6 * inp["BONDSTIFFNESS"][0])])
+    inp["VOLUMECORRECTIONFACTORS"] = np.concatenate([inp["VOLUMECORRECTIONFACTORS"], np.ones(i.size)])
+    inp["nBonds"] += i.size
+    return inp
+
+
+def test_static_solve_ignores_barrier_timeout():
+    """barrier_timeout_s limits the waits of the time stepping alone: a linear solve
+    whose blocks wait for the one with a list of 20 000 entries finishes whatever it is."""
+    inp = with_hubs(bb.beam.build(bb.beam.small(nx=100, ny=10, nz=20)), [5000])
+    g = StaticSolver(inp, law="linear", sc=1.0, barrier_timeout_s=1e-9)
+    st = g.step(-1e-6, tol=1e-30, cg_tol=1e-30, max_cg=8, max_newton=1)
+    assert st.cg_iterations == 8 and st.newton_iterations == 1
+    g.close()
