@@ -333,7 +333,7 @@ constexpr int kCgThreads = 512;   // 16 warps of 128 registers on every SM
 constexpr int kCgWarps = kCgThreads / 32;
 constexpr int kCgRows = 4;         // rows of a warp's gathers in flight
 constexpr int kCgCheck = 8;        // iterations between convergence checks
-constexpr int kCgLaunch = 1024;    // iterations of one launch at most
+constexpr int kCgLaunch = 1024;    // iterations of one launch at most (bbpd_selftest_static_launch changes it)
 // The sums keep the order of 592 groups of 8 warps, whatever the grid: p.Kp goes
 // over the nodes warp by warp (lane l of owner o stands for warp 32 o + l, which
 // takes nodes 32 o + l, 32 o + l + 4736, ...), r.z and r.r over them 32 at a time.
@@ -385,7 +385,7 @@ struct CgArgs {
     unsigned *bar;
     unsigned long long timeout_ns;
     double tol2;                   // stop at r.r <= tol2 * r.r at the start
-    int first, max_cg;
+    int first, max_cg, launch;     // launch: iterations of this launch at most
 };
 enum { CG_MORE = 0, CG_DONE = 1, CG_NONFINITE = 2 };
 
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
         done = A.state[1];
     }
     int state = rr0 > 0 ? CG_MORE : CG_DONE;   // a NaN r.r has nothing to solve either
-    for (int it = 0; it < kCgLaunch && state == CG_MORE; it++) {
+    for (int it = 0; it < A.launch && state == CG_MORE; it++) {
         cg_product(A.g, A.rigE, A.rec, A.y, part1, sm);
         if (!bar.wait()) return;
         const double py = add_groups(part1, pgroups, sm).x;
@@ -688,7 +688,7 @@ struct bbpd_static {
     NodeRec *rec = nullptr;
     double2 *cg_part = nullptr;
     int *cg_state = nullptr;               // state, iterations, error word, barrier arrivals
-    int cg_grid = 0;
+    int cg_grid = 0, cg_launch = kCgLaunch;
     unsigned long long cg_limit_ns = 0;    // of a barrier wait
     double *y = nullptr;
     uint8_t *skip = nullptr;
@@ -718,7 +718,7 @@ int run_cg(bbpd_static *S, double cg_tol, int max_cg, int state[2])
     cudaStream_t st = S->st;
     CgArgs A{S->g, S->rigE, S->rec, S->F, S->Minv, S->skip, S->x, S->d, S->r, S->z, S->y, S->cg_part,
              S->scal, S->cg_state, reinterpret_cast<unsigned *>(S->cg_state + 3), S->cg_limit_ns,
-             cg_tol * cg_tol, 1, max_cg};
+             cg_tol * cg_tol, 1, max_cg, S->cg_launch};
     for (;; A.first = 0) {
         BBPD_CUDA_TRY(cudaMemsetAsync(S->cg_state + 2, 0, 2 * sizeof(int), st));
         void *args[] = {(void *)&A};
@@ -1010,6 +1010,15 @@ extern "C" int bbpd_static_step(bbpd_static *S, double increment, double tol, in
         stats->cg_iterations += cg[1];
         if (cg[0] == CG_NONFINITE) return fail(BBPD_ERR_NONFINITE, "conjugate gradient diverged");
     }
+}
+
+extern "C" int bbpd_selftest_static_launch(bbpd_static *S, int iterations, double limit_s)
+{
+    if (!S || iterations < 1 || !(limit_s >= 0) || limit_s > 1e6)
+        return fail(BBPD_ERR_ARG, "need a solver, iterations >= 1 and 0 <= limit_s <= 1e6");
+    S->cg_launch = iterations;
+    if (limit_s > 0) S->cg_limit_ns = (unsigned long long)(limit_s * 1e9);
+    return BBPD_OK;
 }
 
 extern "C" int bbpd_static_get(bbpd_static *S, int field, double *out)

@@ -592,6 +592,13 @@ int bbpd_last_kernel_ms(bbpd_solver *s, float *ms);
  * wait expires after timeout_s and the kernel returns (the expected outcome). */
 int bbpd_selftest_wait_timeout(double timeout_s);
 
+/* Diagnostic: the linear solves of this static solver run at most `iterations`
+ * conjugate-gradient iterations a launch from now on (1024 until then; the
+ * results do not depend on it) and, where limit_s > 0, give up a barrier wait
+ * after limit_s with BBPD_ERR_TIMEOUT: the solution of that solve is not added
+ * to the positions, and the solver stays usable. */
+int bbpd_selftest_static_launch(bbpd_static *solver, int iterations, double limit_s);
+
 /* Diagnostic: compares the kernels' correctly rounded division by a shared
  * divisor (Markstein's reciprocal and quotient corrections) with IEEE double
  * division on n seeded samples on the device; reports the mismatches of the

@@ -4,6 +4,8 @@ direct sparse solves). The GPU solves each linear system by a preconditioned
 conjugate gradient to a relative residual of 1e-13, so displacements agree to a
 tolerance: 1e-8 of the largest displacement while the beam is elastic, 1e-6
 through softening, with identical softening and broken-bond sets."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -214,3 +216,50 @@ def test_static_solve_ignores_barrier_timeout():
     st = g.step(-1e-6, tol=1e-30, cg_tol=1e-30, max_cg=8, max_newton=1)
     assert st.cg_iterations == 8 and st.newton_iterations == 1
     g.close()
+
+
+def set_launch(g, iterations, limit_s=0.0):
+    L = bb._native.lib()
+    L.bbpd_selftest_static_launch.argtypes = [C.c_void_p, C.c_int, C.c_double]
+    bb._native.check(L.bbpd_selftest_static_launch(g._h, iterations, limit_s))
+
+
+# one launch; launches that end between, at and just past the looks at the residual
+# (every 8 iterations); max_cg on a launch's last iteration, before and after it
+@pytest.mark.parametrize("launch,max_cg", [(1, 200000), (5, 200000), (8, 200000), (17, 200000), (16, 48), (16, 47),
+                                           (16, 49)])
+def test_static_solve_cut_into_launches(launch, max_cg):
+    """A linear solve that goes over several launches carries all of its state from
+    one to the next: the same iterates bit for bit and the same count."""
+    inp = bb.beam.build(bb.beam.small(nx=20, ny=4, nz=6))
+    out = []
+    for n in (1024, launch):
+        g = StaticSolver(inp, law="linear", sc=1.0)
+        set_launch(g, n)
+        st = [g.step(-1e-6, tol=1e-9, cg_tol=1e-13, max_cg=max_cg, max_newton=3) for _ in range(2)]
+        out.append(([(s.cg_iterations, s.newton_iterations, s.residual, s.reaction) for s in st],
+                    g.get("displacement"), g.get("force")))
+        g.close()
+    (a, ua, fa), (b, ub, fb) = out
+    assert a == b and a[0][0] > launch
+    assert np.array_equal(ua, ub) and np.array_equal(fa, fb)
+
+
+def test_static_solve_wait_runs_out():
+    """A barrier wait of the linear solve that runs out is reported, moves nothing
+    and leaves the solver usable."""
+    inp = with_hubs(bb.beam.build(bb.beam.small(nx=100, ny=10, nz=20)), [5000])
+    kw = dict(tol=1e-30, cg_tol=1e-30, max_cg=8, max_newton=1)
+    a, b = (StaticSolver(inp, law="linear", sc=1.0) for _ in range(2))
+    a.step(-1e-6, **kw)
+    set_launch(b, 1024, 1e-9)
+    with pytest.raises(bb.BBPDError) as e:
+        b.step(-1e-6, **kw)
+    assert e.value.status == bb._native.ERR_TIMEOUT
+    moved = (inp["BODYFORCEFLAG"] == 1) & (inp["CONSTRAINTFLAG"] != 1)
+    assert np.array_equal(b.get("displacement") != 0, moved)
+    set_launch(b, 1024, 10.0)
+    b.step(0.0, **kw)
+    assert np.array_equal(a.get("displacement"), b.get("displacement"))
+    a.close()
+    b.close()
