@@ -27,7 +27,8 @@
 // node), which gives the nodal sums their serial order. For the matrix-free
 // products the lists are also laid out in slices of 32 nodes, entry k of the
 // slice's 32 lists side by side (padded to its longest list): the neighbour's id
-// and, per tangent, the bond's stiffness scale, 12 bytes an entry. The bond
+// and, per tangent, the bond's stiffness scale, 12 bytes an entry. Where padding would
+// take most of that (a few nodes with very long lists) they stay lists. The bond
 // vector is the difference of the two nodes' positions, which lie in one record
 // with the direction p. Reductions are fixed-order, so a step is deterministic.
 #include "bbpd_internal.h"
@@ -129,8 +130,8 @@ struct SNodes {
     const int64_t *off;         // [n + 1] list offsets
     const uint32_t *ent;        // directed entries q = 2k + side, by node, in bond order
     const uint32_t *a, *b;      // end nodes of the bonds
-    const int64_t *sptr;        // slots of slice s: [sptr[s], sptr[s + 1])
-    const uint32_t *bond, *col; // bond and neighbour of every slot
+    const int64_t *sptr;        // slots of slice s: [sptr[s], sptr[s + 1]), 32 a row
+    const uint32_t *bond, *col; // bond and neighbour of every slot (LISTS: of every list entry)
     int64_t ns;
     const uint8_t *held;        // per DOF [3 n]: 1 support, 2 prescribed
     int64_t n, nB;
@@ -217,6 +218,18 @@ __global__ void k_slice_fill(const int64_t *__restrict__ off, const uint32_t *__
     }
 }
 
+// The same for lists that stay lists
+__global__ void k_list_fill(const uint32_t *__restrict__ ent, const uint32_t *__restrict__ a, const uint32_t *__restrict__ b,
+                            int64_t m, uint32_t *bond, uint32_t *col)
+{
+    GRID_STRIDE(e, m)
+    {
+        const uint32_t v = ent[e], q = v >> 1;
+        bond[e] = q;
+        col[e] = (v & 1u) ? a[q] : b[q];
+    }
+}
+
 // A node's position and its component of the CG direction p (zero on held and
 // left-out DOFs): 64 bytes, read as a 256-bit and a 128-bit load
 struct __align__(64) NodeRec {
@@ -249,9 +262,9 @@ __global__ void k_static_records(const double *__restrict__ x, int64_t n, NodeRe
 }
 
 __global__ void k_slot_rig(const uint32_t *__restrict__ bond, const double *__restrict__ rig,
-                           const int64_t *__restrict__ slots, double *rigE)
+                           int64_t entries, double *rigE)
 {
-    GRID_STRIDE(e, *slots)
+    GRID_STRIDE(e, entries)
     {
         const uint32_t q = bond[e];
         rigE[e] = q == kNoBond ? 0.0 : rig[q];
@@ -259,21 +272,24 @@ __global__ void k_slot_rig(const uint32_t *__restrict__ bond, const double *__re
 }
 
 // A lane adds its node's list in bond order, four rows of the slice in flight.
+template <bool LISTS>
 __global__ void k_static_precond(SNodes g, const double *__restrict__ rigE, const NodeRec *__restrict__ rec, double *Minv,
                                  uint8_t *skip)
 {
     const int64_t n = g.n;
     GRID_STRIDE(i, n)
     {
-        const int64_t s = i >> 5, rows = (g.sptr[s + 1] - g.sptr[s]) >> 5;
-        const uint32_t *col = g.col + g.sptr[s] + (i & 31);
-        const double *rig = rigE + g.sptr[s] + (i & 31);
+        const int64_t s = i >> 5, rows = LISTS ? g.off[i + 1] - g.off[i] : (g.sptr[s + 1] - g.sptr[s]) >> 5;
+        const int64_t at = LISTS ? g.off[i] : g.sptr[s] + (i & 31);
+        constexpr int kRow = LISTS ? 1 : 32;
+        const uint32_t *col = g.col + at;
+        const double *rig = rigE + at;
         const double xi[3] = {rec[i].x, rec[i].y, rec[i].z};
         double D[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
 #pragma unroll 4
         for (int64_t k = 0; k < rows; k++) {
-            const double r = rig[k * 32];
-            const NodeRec *o = rec + col[k * 32];
+            const double r = rig[k * kRow];
+            const NodeRec *o = rec + col[k * kRow];
             const double c[3] = {o->x - xi[0], o->y - xi[1], o->z - xi[2]};
             for (int u = 0; u < 3; u++)
                 for (int v = 0; v < 3; v++) D[u][v] += r != 0 ? r * c[u] * c[v] : 0.0;
@@ -426,6 +442,7 @@ __device__ __forceinline__ void node_sums(int64_t n, double2 *part, CgShared &sm
 // partials of p.y. A node's sum is 32 partial sums (entries l, l + 32, ... to
 // partial l) folded in a butterfly; warp w of the block takes partials w and
 // w + 16 of the slice's 32 nodes.
+template <bool LISTS>
 __device__ __forceinline__ void cg_product(const SNodes &g, const double *rigE, const NodeRec *rec, double *y, double2 *part,
                                            CgShared &sm)
 {
@@ -448,13 +465,22 @@ __device__ __forceinline__ void cg_product(const SNodes &g, const double *rigE, 
             double h[kCgRows];
             // rows k, k + 32, ... of slice q, if it has them: neighbours and scales
             auto streams = [&](int q, int k) {
-                const int64_t b = __shfl_sync(0xffffffffu, at, q) + lane;
-                const int rows = __shfl_sync(0xffffffffu, len, q);
+                int64_t b;
+                int rows;
+                constexpr int64_t kRow = LISTS ? 1 : 32;
+                if (LISTS) {
+                    const int64_t i = (own + kCgOwners * (m + q)) * 32 + lane;
+                    b = i < n ? g.off[i] : 0;
+                    rows = i < n ? (int)(g.off[i + 1] - b) : 0;
+                } else {
+                    b = __shfl_sync(0xffffffffu, at, q) + lane;
+                    rows = __shfl_sync(0xffffffffu, len, q);
+                }
 #pragma unroll
                 for (int t = 0; t < kCgRows; t++) {
                     const int row = k + 32 * t;
-                    j[t] = row < rows ? __ldg(g.col + b + (int64_t)row * 32) : 0u;
-                    h[t] = row < rows ? __ldg(rigE + b + (int64_t)row * 32) : 0.0;
+                    j[t] = row < rows ? __ldg(g.col + b + row * kRow) : 0u;
+                    h[t] = row < rows ? __ldg(rigE + b + row * kRow) : 0.0;
                 }
             };
             streams(0, w);
@@ -544,6 +570,7 @@ __device__ __forceinline__ void cg_product(const SNodes &g, const double *rigE, 
 // gathers and 12 bytes an entry. 20 000 nodes, 1.0M bonds, B200: 109 us an
 // iteration with six kernels, 33 here.
 // Warps with equal runs of rows and sums in any order took 22.
+template <bool LISTS>
 __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
 {
     extern __shared__ __align__(16) unsigned char cg_smem[];
@@ -586,7 +613,7 @@ __global__ void __launch_bounds__(kCgThreads, 1) k_cg(CgArgs A)
     }
     int state = rr0 > 0 ? CG_MORE : CG_DONE;   // a NaN r.r has nothing to solve either
     for (int it = 0; it < A.launch && state == CG_MORE; it++) {
-        cg_product(A.g, A.rigE, A.rec, A.y, part1, sm);
+        cg_product<LISTS>(A.g, A.rigE, A.rec, A.y, part1, sm);
         if (!bar.wait()) return;
         const double py = add_groups(part1, pgroups, sm).x;
         // delta += alpha p, r -= alpha y, z = M^-1 r
@@ -688,6 +715,9 @@ struct bbpd_static {
     NodeRec *rec = nullptr;
     double2 *cg_part = nullptr;
     int *cg_state = nullptr;               // state, iterations, error word, barrier arrivals
+    bool lists = false;                    // the solve's entries lie in lists, not in slices
+    int64_t entries = 0;                   // of bond, col and rigE
+    void (*cg)(CgArgs) = nullptr;
     int cg_grid = 0, cg_launch = kCgLaunch;
     unsigned long long cg_limit_ns = 0;    // of a barrier wait
     double *y = nullptr;
@@ -722,7 +752,7 @@ int run_cg(bbpd_static *S, double cg_tol, int max_cg, int state[2])
     for (;; A.first = 0) {
         BBPD_CUDA_TRY(cudaMemsetAsync(S->cg_state + 2, 0, 2 * sizeof(int), st));
         void *args[] = {(void *)&A};
-        BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_cg, dim3(S->cg_grid), dim3(kCgThreads), args, sizeof(CgShared), st));
+        BBPD_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)S->cg, dim3(S->cg_grid), dim3(kCgThreads), args, sizeof(CgShared), st));
         int h[3];
         BBPD_CUDA_TRY(cudaMemcpyAsync(h, S->cg_state, sizeof(h), cudaMemcpyDeviceToHost, st));
         BBPD_CUDA_TRY(cudaStreamSynchronize(st));
@@ -934,17 +964,26 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
         if (tmp) cudaFreeAsync(tmp, st);
         if (e != cudaSuccess) return fail(BBPD_ERR_CUDA, "static solver slices: %s", cudaGetErrorString(e));
     }
-    TRY(S->alloc(&bond, slots));
-    TRY(S->alloc(&col, slots));
-    TRY(S->alloc(&S->rigE, slots));
-    k_slice_fill<<<blocks_for(32 * ns), kThreads, 0, st>>>(off, ent, da, db, n, ns, sptr, bond, col);
+    // Slices where padding takes at most three quarters of them (a beam's take under
+    // 1.3 times its entries): 16 bytes a slot, read a row at a time. Beyond, the memory
+    // would be the longest lists' 32-fold: 20 000 nodes, 64 of them bonded to all
+    // others, took 910 MB against 306 with lists, and 400 iterations 275 ms against
+    // 172 (552 with six kernels an iteration).
+    S->lists = slots > 4 * m;
+    S->entries = S->lists ? m : slots;
+    TRY(S->alloc(&bond, S->entries));
+    TRY(S->alloc(&col, S->entries));
+    TRY(S->alloc(&S->rigE, S->entries));
+    if (S->lists) k_list_fill<<<blocks_for(m), kThreads, 0, st>>>(ent, da, db, m, bond, col);
+    else k_slice_fill<<<blocks_for(32 * ns), kThreads, 0, st>>>(off, ent, da, db, n, ns, sptr, bond, col);
     TRY(launch_check());
     int nsm = 0, occ = 0, coop = 0;
     BBPD_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
     BBPD_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
     if (!coop) return fail(BBPD_ERR_UNSUPPORTED, "device lacks cooperative launch");
-    BBPD_CUDA_TRY(cudaFuncSetAttribute(k_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgShared)));
-    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg, kCgThreads, sizeof(CgShared)));
+    S->cg = S->lists ? k_cg<true> : k_cg<false>;
+    BBPD_CUDA_TRY(cudaFuncSetAttribute(S->cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgShared)));
+    BBPD_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, S->cg, kCgThreads, sizeof(CgShared)));
     if (occ < 1) return fail(BBPD_ERR_CUDA, "kernel cannot be resident");
     // a block for every owner with slices
     S->cg_grid = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)nsm, (int64_t)kCgOwners, ns}));
@@ -1002,8 +1041,9 @@ extern "C" int bbpd_static_step(bbpd_static *S, double increment, double tol, in
         if (it == max_newton) return BBPD_OK;   // not converged: stats say so
         // K delta = F on the free DOFs by PCG, x += delta
         k_static_records<<<blocks_for(n), kThreads, 0, st>>>(S->x, n, S->rec);
-        k_slot_rig<<<blocks_for(2 * S->nB), kThreads, 0, st>>>(S->g.bond, S->b.rig, S->g.sptr + S->g.ns, S->rigE);
-        k_static_precond<<<blocks_for(n), kThreads, 0, st>>>(S->g, S->rigE, S->rec, S->Minv, S->skip);
+        k_slot_rig<<<blocks_for(S->entries), kThreads, 0, st>>>(S->g.bond, S->b.rig, S->entries, S->rigE);
+        (S->lists ? k_static_precond<true> : k_static_precond<false>)<<<blocks_for(n), kThreads, 0, st>>>(
+            S->g, S->rigE, S->rec, S->Minv, S->skip);
         TRY(launch_check());
         int cg[2] = {CG_DONE, 0};
         TRY(run_cg(S, cg_tol, max_cg, cg));

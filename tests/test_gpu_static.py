@@ -263,3 +263,33 @@ def test_static_solve_wait_runs_out():
     assert np.array_equal(a.get("displacement"), b.get("displacement"))
     a.close()
     b.close()
+
+
+# 4 lists of 480 among lists of 18, padding more than three quarters of the slices
+# (lists stay lists); 4 among lists of 122 (slices); every node bonded to all others
+@pytest.mark.parametrize("hf,hubs", [(1.5, 4), (3.015, 4), (1.5, 480)])
+def test_static_solve_uneven_lists_vs_oracle(hf, hubs):
+    inp = with_hubs(bb.beam.build(bb.beam.small(nx=20, ny=4, nz=6, horizon_factor=hf)),
+                    list(range(0, 480, 480 // hubs)))
+    g = StaticSolver(inp, law="linear", sc=1.0)
+    o = StaticOracle(inp, law="linear", sc=1.0)
+    for step in range(2):
+        sg = g.step(-1e-6, tol=1e-9, **CG)
+        so = o.step(-1e-6, tol=1e-9)
+        assert sg.converged and so["converged"], (step, sg.residual, sg.reaction)
+        ug, uo = g.get("displacement"), o.get("displacement")
+        assert np.abs(ug - uo).max() <= 1e-8 * np.abs(uo).max(), step
+    g.close()
+
+
+def test_static_uneven_lists_memory():
+    """A few nodes with very long lists do not make every list as long: some 130
+    bytes a bond and 300 a node, not 16 bytes for 32 times the longest lists."""
+    import torch
+    inp = with_hubs(bb.beam.build(bb.beam.small(nx=100, ny=10, nz=20)), list(range(16, 20000, 313)))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    g = StaticSolver(inp, law="linear", sc=1.0)
+    used = free - torch.cuda.mem_get_info()[0]
+    g.close()
+    assert used <= 200 * inp["nBonds"] + 500 * inp["nNodes"], used
