@@ -603,8 +603,9 @@ extern "C" int bbpd_dev_calculatedampingcoefficient(const double *F, const doubl
     return rc;
 }
 
-extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, int nChunks,
-                                      void *stream, bbpd_nodal_plan **out)
+// narrow: 32-bit entries
+static int plan_create(const double *bl, int64_t nB, int64_t nN, int nChunks, void *stream, bool narrow,
+                       bbpd_nodal_plan **out)
 {
     if (!out || nB < 0 || nN < 0 || nChunks < 1 || nN >= (int64_t)1 << 31)
         return fail(BBPD_ERR_ARG, "bad plan arguments");
@@ -619,12 +620,11 @@ extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, 
     int *bad = nullptr;
     void *tmp = nullptr;
     size_t tmpb = 0;
-    const bool narrow = ne < (int64_t)1 << 31;   // the top bit is the chunk flag
     cudaError_t e = cudaSuccess;
 #define PLAN_TRY(x) do { e = (x); if (e != cudaSuccess) goto fail_; } while (0)
     PLAN_TRY(cudaMalloc(&p->rp, sizeof(int64_t) * (size_t)(nN + 1)));
     if (narrow) PLAN_TRY(cudaMalloc(&p->ent32, sizeof(uint32_t) * (size_t)(ne > 0 ? ne : 1)));
-    else PLAN_TRY(cudaMalloc(&p->ent64, sizeof(uint64_t) * (size_t)ne));
+    else PLAN_TRY(cudaMalloc(&p->ent64, sizeof(uint64_t) * (size_t)(ne > 0 ? ne : 1)));
     PLAN_TRY(cudaMalloc(&cnt, sizeof(int32_t) * (size_t)(nN + 1)));
     PLAN_TRY(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (size_t)(nN + 1), st));
     PLAN_TRY(cudaMalloc(&bad, sizeof(int)));
@@ -683,6 +683,18 @@ fail_:
     return fail(e == cudaErrorMemoryAllocation ? BBPD_ERR_OOM : BBPD_ERR_CUDA, "nodal plan: %s",
                 cudaGetErrorString(e));
 #undef PLAN_TRY
+}
+
+extern "C" int bbpd_nodal_plan_create(const double *bl, int64_t nB, int64_t nN, int nChunks, void *stream,
+                                      bbpd_nodal_plan **out)
+{
+    return plan_create(bl, nB, nN, nChunks, stream, nB < (int64_t)1 << 30, out);   // the top bit is the chunk flag
+}
+
+extern "C" int bbpd_selftest_nodal_plan_create_wide(const double *bl, int64_t nB, int64_t nN, int nChunks, void *stream,
+                                                    bbpd_nodal_plan **out)
+{
+    return plan_create(bl, nB, nN, nChunks, stream, false, out);
 }
 
 extern "C" int bbpd_nodal_plan_destroy(bbpd_nodal_plan *p)

@@ -592,6 +592,11 @@ int bbpd_last_kernel_ms(bbpd_solver *s, float *ms);
  * wait expires after timeout_s and the kernel returns (the expected outcome). */
 int bbpd_selftest_wait_timeout(double timeout_s);
 
+/* Diagnostic: bbpd_nodal_plan_create with the 64-bit entries that it takes from
+ * 2^30 bonds on, for any number of bonds. */
+int bbpd_selftest_nodal_plan_create_wide(const double *bondlist_dev, int64_t nBonds,
+        int64_t nNodes, int nChunks, void *stream, bbpd_nodal_plan **plan);
+
 /* Diagnostic: the linear solves of this static solver run at most `iterations`
  * conjugate-gradient iterations a launch from now on (1024 until then; the
  * results do not depend on it) and, where limit_s > 0, give up a barrier wait

@@ -142,6 +142,32 @@ def test_nodalforces_short_lists(nN, ring, hub, T):
     assert same(F, Fo)
 
 
+@pytest.mark.parametrize("nN,ring,T", [(7, 3, 8), (129, 40, 1), (129, 40, 8), (65536, 3, 8)])
+def test_nodalforces_wide_entries(nN, ring, T):
+    """The 64-bit entries that bond lists of 2^30 bonds take, on small lists: both
+    summing kernels give the 32-bit entries' forces bit for bit, and the oracle's."""
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(nN)
+    i = np.tile(np.arange(nN), ring)
+    bl = np.asfortranarray(np.stack([i, (i + 1) % nN], 1)[rng.permutation(i.size)] + 1.0)
+    nB = len(bl)
+    f = [rng.normal(0, 1e3, nB) for _ in range(3)]
+    Fo = np.asfortranarray(rng.normal(0, 1, (nN, 3)))
+    L, p = bb._native.lib(), lambda t: C.c_void_p(t.data_ptr())
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a.T)).cuda()
+    dbl, df, out = dev(bl), [dev(a) for a in f], []
+    for create in (L.bbpd_nodal_plan_create, L.bbpd_selftest_nodal_plan_create_wide):
+        F, plan = dev(Fo), C.c_void_p()
+        bb._native.check(create(p(dbl), C.c_int64(nB), C.c_int64(nN), T, None, C.byref(plan)))
+        bb._native.check(L.bbpd_dev_calculatenodalforces(plan, p(F), *map(p, df), None))
+        torch.cuda.synchronize()
+        L.bbpd_nodal_plan_destroy(plan)
+        out.append(F.cpu().numpy().T)
+    po.lib().orc_nodalforces_chunked(nB, nN, P(bl), P(Fo), P(f[0]), P(f[1]), P(f[2]), T)
+    assert same(out[0], Fo) and same(out[1], Fo)
+
+
 def test_eulercromer_golden():
     g = gold("eulercromer")
     nN = g["F"].shape[0]
