@@ -724,7 +724,9 @@ __device__ __forceinline__ bool group_fast(const Dev &d, const Group<CID> &G, in
                                            const double4 *xa, double xi, double yi, double zi, double (&fx)[4],
                                            double (&fy)[4], double (&fz)[4])
 {
-    if (__any_sync(0xffffffffu, G.s != 0) || !safe) return false;
+    // one answer for the warp, which votes again below: `safe` is read lane by lane, and
+    // another block may clear it in between
+    if (__any_sync(0xffffffffu, (G.s != 0) | !safe)) return false;
     Rec r[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) load_rec(d, xa, group_w(G, q), G.cid(q), r[q]);
