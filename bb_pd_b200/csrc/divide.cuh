@@ -4,44 +4,22 @@
 // theorems), as also presented in Cornea, Harrison & Tang, "Scientific
 // Computing on Itanium-based Systems", 2002, ch. 8.
 //
-//   recip_rn(b):  y0 = hardware reciprocal approximation (rcp.approx.ftz.f64),
-//                 Newton-Raphson y <- y + y (1 - b y) until within one ulp, then
-//                 one more correction step, which yields RN(1/b) for every b
-//                 whose significand is not all ones (those are reported).
 //   quot_rn(a, b, y):  with y = RN(1/b): q0 = RN(a y), r = a - q0 b (exact by
 //                 fused multiply-add), q = RN(q0 + r y) = RN(a / b).
 //
+// The reciprocal of an undeformed length is an IEEE division on the host (the bond
+// dictionary), that of a deformed length comes with its square root
+// (sqrt_recip_rn).
+//
 // Preconditions (no underflow or overflow in any step): b and a / b normal and
-// well inside the exponent range, a not -0. The kernels use these only when
+// well inside the exponent range, a not -0. The kernels use this only when
 // every coordinate is +0 or of magnitude in [2^-100, 2^100] and L0 lies in the
 // same range; outside it they fall back to IEEE division. bbpd_selftest_division
-// compares both against IEEE `/` bit for bit on the device.
+// compares it, with both kinds of reciprocal, against IEEE `/` bit for bit on the
+// device.
 #pragma once
 
 namespace bbpd {
-
-__device__ __forceinline__ double rcp_approx(double b)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    return y;
-}
-
-// RN(1/b) for normal positive b in [2^-200, 2^200]; ok = false when the low
-// 32 bits of the significand are all ones, which includes the all-ones
-// significand (the one case the final step does not cover).
-__device__ __forceinline__ double recip_rn(double b, bool &ok)
-{
-    double y = rcp_approx(b);
-    double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, e, y);
-    ok = __double2loint(b) != -1;
-    return y;
-}
 
 // RN(a / b) given y = RN(1/b), for a = +0 or |a / b| normal (see
 // preconditions). An exact q0 leaves r = +0 and q0 unchanged.
@@ -58,8 +36,9 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y)
 // RNC'6, 2004. With y0 ~ 1/sqrt(x), g = x y0 and h = y0/2 converge together to
 // sqrt(x) and 1/(2 sqrt(x)): r = 1/2 - g h, g <- g + g r, h <- h + h r. Two
 // rounds leave g and h a few units of 2^-53 off, whatever the seed's last bits
-// are; then d = x - g^2 and RN(g + d h) is the square root, and 2h starts the
-// Newton steps of recip_rn two rounds on.
+// are; then d = x - g^2 and L = RN(g + d h) is the square root. Two Newton-Raphson
+// steps y <- y + y (1 - L y) from y = 2h give RN(1/L) for every L whose significand
+// is not all ones (the reciprocal theorem).
 //
 // Error of g + d h before its rounding, relative, with g and h within
 // 2.5 2^-53: second order 3.1 2^-106, h's error on d h 6.2 2^-106, rounding of
@@ -78,8 +57,9 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y)
 // 121.7 us, 1.28M nodes 865 -> 818 us, eight beams in a batch 270 -> 262 us.
 //
 // ok = false where x is zero, negative, infinite, NaN or outside
-// [2^-700, 2^700), and for the significand of recip_rn's ok: the caller takes
-// IEEE operations then.
+// [2^-700, 2^700), and where the low 32 bits of L are all ones, which includes the
+// significand that the last step does not cover: the caller takes IEEE operations
+// then.
 __device__ __forceinline__ double rsqrt_approx(double x)
 {
     double y;

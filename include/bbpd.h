@@ -605,10 +605,12 @@ int bbpd_selftest_nodal_plan_create_wide(const double *bondlist_dev, int64_t nBo
 int bbpd_selftest_static_launch(bbpd_static *solver, int iterations, double limit_s);
 
 /* Diagnostic: compares the kernels' correctly rounded division by a shared
- * divisor (Markstein's reciprocal and quotient corrections) with IEEE double
- * division on n seeded samples on the device; reports the mismatches of the
- * reciprocal and of the quotients, the samples compared, and the largest
- * relative error of the hardware reciprocal approximation. */
+ * divisor (Markstein's quotient correction) with IEEE double division on n
+ * seeded samples on the device, with the reciprocals that the kernels use: the
+ * bond dictionary's IEEE division, and the one that comes with a square root.
+ * Reports the mismatches of the reciprocal and of the quotients, the samples
+ * compared, and the largest relative error of the hardware reciprocal
+ * approximation. */
 int bbpd_selftest_division(int64_t n, uint64_t seed, int64_t *recip_mismatches,
                            int64_t *quot_mismatches, int64_t *samples,
                            double *rcp_approx_max_relerr);
