@@ -129,7 +129,6 @@ __global__ void k_static_bonds(SBonds s, const double *__restrict__ x, int64_t n
 struct SNodes {
     const int64_t *off;         // [n + 1] list offsets
     const uint32_t *ent;        // directed entries q = 2k + side, by node, in bond order
-    const uint32_t *a, *b;      // end nodes of the bonds
     const int64_t *sptr;        // slots of slice s: [sptr[s], sptr[s + 1]), 32 a row
     const uint32_t *bond, *col; // bond and neighbour of every slot (LISTS: of every list entry)
     int64_t ns;
@@ -997,8 +996,6 @@ extern "C" int bbpd_static_create(const bbpd_problem *pb, const bbpd_params *prm
     TRY(S->alloc(&S->cg_state, 4));
     S->g.off = off;
     S->g.ent = ent;
-    S->g.a = da;
-    S->g.b = db;
     S->g.sptr = sptr;
     S->g.bond = bond;
     S->g.col = col;
