@@ -858,7 +858,7 @@ __device__ __forceinline__ double3 entry_general_x(const Dev &d, int64_t e, uint
 //
 // The fast path of one group, without branches; returns the mask of the slots
 // that need the general path. Padding slots name node 0 and dictionary entry 0
-// (see group_fast).
+// (see group_forces).
 template <int LAW, class CID, int SCE>
 __device__ __forceinline__ unsigned group_fast_x(const Dev &d, const Group<CID> &G, int64_t e0, const float4 *urh,
                                                  const float2 *url, float4 ui, float2 li, float (&fx)[4],
@@ -2547,11 +2547,17 @@ kernel_t pick_kernel(int law, int scheme, int prec, bool wide, bool sce, bool sp
 // round trip costs more than it saves. us per step on B200, step_kernel against
 // split_kernel, ADR: 23 slices 34.8 / 14.7, 203: 41.9 / 19.3, 625: 42.0 / 33.1,
 // 1080: 44.3 / 48.9, 1792: 70.7 / 73.7; Euler-Cromer: 23: 28.8 / 8.7, 203: 32.5 /
-// 12.2, 625: 32.8 / 24.0, 1080: 34.4 / 37.0.
+// 12.2, 625: 32.8 / 24.0, 1080: 34.4 / 37.0. The line is for a beam by itself. split_kernel
+// takes the whole GPU for one beam, so beams stepped at once, each on its solver's
+// stream, gain less or lose against a warp per slice: four and eight ADR beams of
+// 203 slices 18.8 us a beam-step (14.4 and 8.0 with step_kernel), of 625 slices 35.5
+// (28.3 and 24.9); Euler-Cromer 11.6 (11.0 and 7.5) and 24 (28 and 23). Below 148
+// slices in all it is the faster one there too (eight of 23: 3.8 against 6.1). A batch
+// takes 8.7 us for a beam of eight of 203 slices.
 int64_t split_limit(int nsm) { return std::min<int64_t>(kSplitMax, 6 * (int64_t)nsm); }
 
-// Blocks of the kernels that give a slice to a warp: no more than the slices
-// need, but the same number on every SM. With just enough of them (224 for 1792
+// Blocks of the kernels that give a slice to a warp: what the slices need, rounded up
+// to the same number on every SM. With just enough of them (224 for 1792
 // slices) some SMs held two and some one, and the step took as long as the
 // fuller ones: 56 us with 296 against 67 (ADR), 45 against 56 (Euler-Cromer).
 // One block per SM where that gives every slice a warp: 42 against 53 us at 1080.
