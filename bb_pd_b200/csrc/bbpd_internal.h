@@ -37,7 +37,8 @@ int require_device();
 // device (freed with cudaFreeAsync). The default pool gives everything back to
 // the driver at each synchronisation, so a call that ends with one mapped its
 // temporaries anew every time; this pool keeps up to kScratchKeep bytes until
-// release_scratch (bbpd_release_mirrors) or process exit.
+// release_scratch (bbpd_release_mirrors) or process exit. Where the default pool
+// keeps that much already, the temporaries come from there.
 constexpr uint64_t kScratchKeep = (uint64_t)256 << 20;
 cudaError_t scratch_malloc(void **p, size_t bytes, cudaStream_t st);
 void release_scratch();
